@@ -35,6 +35,7 @@ namespace {
 
 constexpr int kCgThreads = 1024;
 constexpr int kMultiThreads = 256;
+constexpr size_t kMgSharedBytes = (sizeof(MgShared) + 15) & ~(size_t)15;
 
 // The solver body, run by `nblk` blocks of which this is block `blk` (a whole grid for one scene, or a
 // block range of a multi-scene launch, see k_multi_cg); every barrier and reduction spans those blocks.
@@ -203,12 +204,20 @@ __global__ void __launch_bounds__(kCgThreads, 1) k_cg(SceneView v, CgWork w, CgP
 }
 
 // The same solve with the multigrid-preconditioned inner loop (fe_mg_body.cuh).
+// FEW: threads per tile where there are few tiles (fe_mg_body.cuh).  Grids with fewer tiles than blocks are solved by as
+// many blocks as there are tiles; the others leave at once.
+template <int FEW>
 __global__ void __launch_bounds__(kCgThreads, 1) k_mgcg(SceneView v, CgWork w, MgWork mg, CgParams prm)
 {
-    __shared__ SolverSmem smem;
-    cluster_begin(w, smem.sh);
-    mg_body(smem, v, w, mg, prm, blockIdx.x, gridDim.x);
-    solver_exit(w, gridDim.x);
+    __shared__ MgShared ms;
+    extern __shared__ __align__(16) unsigned char mg_dynamic[];
+    cluster_begin(w, ms.sh);
+    const int tiles = tiles_of(v.g.nx) * tiles_of(v.g.ny) * tiles_of(v.g.nz);
+    const int nblk = w.cluster > 1 ? (int)gridDim.x : min((int)gridDim.x, tiles);
+    if ((int)blockIdx.x < nblk) {
+        mg_body<FEW, 256>(ms, reinterpret_cast<MgTeam*>(mg_dynamic), v, w, mg, prm, blockIdx.x, nblk);
+        solver_exit(w, nblk);
+    }
     cluster_end(w);
 }
 
@@ -231,9 +240,14 @@ __global__ void __launch_bounds__(kMultiThreads, 3) k_multi_cg(MultiCgScene* __r
     prm.stats_cap = m.work.stats_cap;
     int its = 0, fluid = 0;
     const int blk = (int)blockIdx.x - m.block_start;
-    __shared__ SolverSmem smem;
-    if (m.use_mg) mg_body(smem, m.view, m.work, m.mg, prm, blk, m.block_count, &its, &fluid);
-    else cg_body(smem, m.view, m.work, prm, blk, m.block_count, &its, &fluid);
+    extern __shared__ __align__(16) unsigned char multi_dynamic[];
+    if (m.use_mg) {
+        MgShared& ms = *reinterpret_cast<MgShared*>(multi_dynamic);
+        mg_body<kMultiThreads, kMultiThreads>(ms, reinterpret_cast<MgTeam*>(multi_dynamic + kMgSharedBytes), m.view, m.work,
+                                              m.mg, prm, blk, m.block_count, &its, &fluid);
+    } else {
+        cg_body(*reinterpret_cast<SolverSmem*>(multi_dynamic), m.view, m.work, prm, blk, m.block_count, &its, &fluid);
+    }
     solver_exit(m.work, m.block_count);
     if (blk == 0 && threadIdx.x == 0) {  // read by the next solve's k_multi_partition
         m.last_its = its;
@@ -320,12 +334,17 @@ cudaError_t set_solver_barrier_limits(unsigned long long spin_limit, unsigned ex
     return cudaMemcpyToSymbol(c_extra_arrivals, &extra_arrivals, sizeof(extra_arrivals));
 }
 
+// Dynamic shared memory of k_multi_cg: either body's.
+static size_t multi_smem() { return std::max(sizeof(SolverSmem), kMgSharedBytes + mg_dynamic_smem(kMultiThreads)); }
+
 cudaError_t multi_cg_capacity(int device, int* max_blocks, int* threads)
 {
     int sms = 0, per_sm = 0;
     cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_multi_cg, kMultiThreads, 0);
+    e = cudaFuncSetAttribute(k_multi_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)multi_smem());
+    if (e != cudaSuccess) return e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_multi_cg, kMultiThreads, multi_smem());
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorCooperativeLaunchTooLarge;
     *max_blocks = sms * per_sm;
@@ -340,6 +359,7 @@ cudaError_t launch_multi_cg(MultiCgScene* scenes, int S, int total_blocks, cudaS
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)total_blocks);
     cfg.blockDim = dim3((unsigned)kMultiThreads);
+    cfg.dynamicSmemBytes = multi_smem();
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -351,6 +371,9 @@ cudaError_t launch_multi_cg(MultiCgScene* scenes, int S, int total_blocks, cudaS
     return e;
 }
 
+using MgcgKernel = void (*)(SceneView, CgWork, MgWork, CgParams);
+static MgcgKernel mgcg_kernel(int threads) { return threads < 512 ? k_mgcg<256> : k_mgcg<512>; }
+
 cudaError_t cg_prepare(CgWork& w, int device, int threads, int cluster)
 {
     if (threads != 256 && threads != 512 && threads != 1024) return cudaErrorInvalidValue;
@@ -361,7 +384,9 @@ cudaError_t cg_prepare(CgWork& w, int device, int threads, int cluster)
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg, threads, 0);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_mg, k_mgcg, threads, 0);
+    e = cudaFuncSetAttribute(mgcg_kernel(threads), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mg_dynamic_smem(threads));
+    if (e != cudaSuccess) return e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_mg, mgcg_kernel(threads), threads, mg_dynamic_smem(threads));
     if (e != cudaSuccess) return e;
     // persistent blocks: as many per SM as fill 1024 threads, all co-resident (a cooperative launch)
     const int want = kCgThreads / threads;
@@ -375,6 +400,7 @@ cudaError_t cg_prepare(CgWork& w, int device, int threads, int cluster)
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)(clusters * cluster));
             cfg.blockDim = dim3((unsigned)threads);
+            cfg.dynamicSmemBytes = kind == 0 ? 0 : mg_dynamic_smem(threads);
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = (unsigned)cluster;
@@ -383,7 +409,7 @@ cudaError_t cg_prepare(CgWork& w, int device, int threads, int cluster)
             cfg.attrs = attr;
             cfg.numAttrs = 1;
             int n = 0;
-            e = kind == 0 ? cudaOccupancyMaxActiveClusters(&n, k_cg, &cfg) : cudaOccupancyMaxActiveClusters(&n, k_mgcg, &cfg);
+            e = kind == 0 ? cudaOccupancyMaxActiveClusters(&n, k_cg, &cfg) : cudaOccupancyMaxActiveClusters(&n, mgcg_kernel(threads), &cfg);
             if (e != cudaSuccess) return e;
             clusters = std::min(clusters, n);
         }
@@ -442,6 +468,7 @@ cudaError_t launch_mgcg(const SceneView& v, const CgWork& w, const MgWork& mg, d
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)w.blocks);
     cfg.blockDim = dim3((unsigned)w.threads);
+    cfg.dynamicSmemBytes = mg_dynamic_smem(w.threads);
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -452,7 +479,7 @@ cudaError_t launch_mgcg(const SceneView& v, const CgWork& w, const MgWork& mg, d
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = w.cluster > 1 ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k_mgcg, v, w, mg, prm);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, mgcg_kernel(w.threads), v, w, mg, prm);
     count_launch();
     return e;
 }

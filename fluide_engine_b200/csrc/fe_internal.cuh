@@ -308,18 +308,18 @@ cudaError_t set_solver_barrier_limits(unsigned long long spin_limit, unsigned ex
 // vectors are the solver's own (CgWork); level l >= 1 halves every axis of level l-1 (rounding up) until
 // the largest axis is <= 8, and that last level is solved by one block.
 constexpr int kMaxMgLevels = 12;
-// FE_PRESSURE_AUTO picks the multigrid solver from this many grid cells on.  Measured on B200 over whole
-// 240-substep dam-break runs (ms per solve, plain / multigrid): 24^3 0.36 / 0.39, 32^3 0.46 / 0.39, 40^3 0.55 /
-// 0.52, 48^3 0.64 / 0.63, 64^3 0.85 / 0.67, 96^3 - / 1.27, 128^3 3.24 / 1.91; at 256^3 the multigrid one wins by
-// 8x (the plain CG streams its vectors from HBM about 1,000 times per solve).
-constexpr size_t kMgAutoCells = (size_t)1 << 15;
+// FE_PRESSURE_AUTO picks the multigrid solver from this many grid cells on (grids of at most 8 cells per axis have no
+// hierarchy and keep the plain one).  Measured on B200, dam break to 1e-6 (us per solve, plain / multigrid): 12^3 211 /
+// 178, 16^3 285 / 190, 20^3 348 / 244, 24^3 426 / 266, 28^3 479 / 258, 32^3 539 / 256, 40^3 635 / 309; 64^3 and above the
+// plain one takes two to ten times as long.
+constexpr size_t kMgAutoCells = (size_t)1 << 10;
 struct MgLevel {
     int nx, ny, nz;
     float ih2[3];      // 1 / h_l^2 per axis, h_l = 2^l h
-    uint8_t* mask;     // l >= 1: 1 where some child cell holds fluid
+    float* inv;        // l >= 1: 1 / D of the level's operator, 0 where the cell is outside the system
     float* r;          // l >= 1: restricted residual
     float* z;          // l >= 1: correction
-    float* t;          // l >= 1: scratch: the level's residual going down, its pre-smoothed correction going up
+    float* t;          // l >= 1: the cells' fluid fractions (solver setup), then the pre-smoothed correction
 };
 struct MgWork {
     int levels;        // levels in use (0 or 1: no hierarchy, the plain CG solves)

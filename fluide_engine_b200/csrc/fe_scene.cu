@@ -346,11 +346,11 @@ fe_status ensure_mg(fe_scene* s)
     for (int l = 1; l < levels; ++l) {
         MgLevel& M = lv[l];
         const size_t cells = (size_t)M.nx * M.ny * M.nz;
-        FE_CUDA(dalloc(L, &M.mask, cells, dev, st));
+        FE_CUDA(dalloc(L, &M.inv, cells, dev, st));
         FE_CUDA(dalloc(L, &M.r, cells, dev, st));
         FE_CUDA(dalloc(L, &M.z, cells, dev, st));
         FE_CUDA(dalloc(L, &M.t, cells, dev, st));
-        FE_CUDA(cudaMemsetAsync(M.mask, 0, cells, st));
+        FE_CUDA(cudaMemsetAsync(M.inv, 0, cells * sizeof(float), st));
         FE_CUDA(cudaMemsetAsync(M.r, 0, cells * sizeof(float), st));
         FE_CUDA(cudaMemsetAsync(M.z, 0, cells * sizeof(float), st));
         FE_CUDA(cudaMemsetAsync(M.t, 0, cells * sizeof(float), st));

@@ -343,10 +343,6 @@ struct SolverSmem {
     double sh[kShDoubles];                 // block reductions, then the cluster pre-reduction's words
     uint32_t s_warp[32];                   // compaction counts
     uint32_t s_list[kListCache];           // cached FLUID-list entries
-    float cz[2][kCoarseMaxCells];          // multigrid: coarsest-level correction (ping-pong)
-    float cr[kCoarseMaxCells];             // multigrid: coarsest-level right-hand side
-    float cw[kCoarseMaxCells];             // multigrid: coarsest-level omega / diagonal (0 outside the mask)
-    uint8_t cb[kCoarseMaxCells];           // multigrid: coarsest-level in-domain neighbour bits
 };
 
 // Solver setup shared by the persistent solvers, run by `nblk` blocks of which this is block `blk`: zeroes
@@ -368,10 +364,10 @@ struct SolverSetup {
 // 0 for non-FLUID cells.  A FLUID cell enclosed by BOUNDRY cells and walls has an all-zero row in the reference's
 // system: nothing couples to it and its pressure reaches no face (ApplyPressure skips faces toward BOUNDRY), so it
 // is left out of the solve with pressure 0 instead of holding the residual at |b| for every iteration.
-__device__ __forceinline__ uint32_t solve_mask(const uint8_t* __restrict__ marks, int c, int nx, int ny, int nz)
+__device__ __forceinline__ uint32_t solve_mask(const uint8_t* __restrict__ marks, int c, int i, int j, int k, int nx, int ny,
+                                               int nz)
 {
     if (marks[c] != FE_CELL_FLUID) return 0u;
-    const int i = c % nx, j = (c / nx) % ny, k = c / (nx * ny);
     const size_t sxy1 = (size_t)nx * ny;
     return (i > 0 && marks[c - 1] != FE_CELL_BOUNDRY ? kXm : 0u) |
            (i + 1 < nx && marks[c + 1] != FE_CELL_BOUNDRY ? kXp : 0u) |
@@ -379,6 +375,11 @@ __device__ __forceinline__ uint32_t solve_mask(const uint8_t* __restrict__ marks
            (j + 1 < ny && marks[c + nx] != FE_CELL_BOUNDRY ? kYp : 0u) |
            (k > 0 && marks[c - sxy1] != FE_CELL_BOUNDRY ? kZm : 0u) |
            (k + 1 < nz && marks[c + sxy1] != FE_CELL_BOUNDRY ? kZp : 0u);
+}
+
+__device__ __forceinline__ uint32_t solve_mask(const uint8_t* __restrict__ marks, int c, int nx, int ny, int nz)
+{
+    return solve_mask(marks, c, c % nx, (c / nx) % ny, c / (nx * ny), nx, ny, nz);
 }
 
 __device__ __forceinline__ bool solver_setup(const SceneView& v, const CgWork& w, const int blk, const int nblk,
