@@ -112,11 +112,11 @@ __device__ __forceinline__ void load_vertex(const MeshView& m, int64_t id, doubl
 }
 
 // The winding sum of TriangleMesh::IsInside (3d/triangle_mesh.cpp:120-163): atan2(det(A, B, C), k) over the
-// triangles, A, B, C the vertices relative to the point (half the solid angle each).
-__device__ __forceinline__ double winding_sum(const MeshView& m, const double pt[3])
+// triangles, A, B, C the vertices relative to the point (half the solid angle each); triangles first, first + step, ...
+__device__ __forceinline__ double winding_sum(const MeshView& m, const double pt[3], uint64_t first = 0, uint64_t step = 1)
 {
     double ret = 0.0;
-    for (uint64_t t = 0; t < m.nt; ++t) {
+    for (uint64_t t = first; t < m.nt; t += step) {
         double A[3], B[3], C[3];
         load_vertex(m, __ldg(m.T + 4 * t), A);
         load_vertex(m, __ldg(m.T + 4 * t + 1), B);

@@ -15,8 +15,12 @@
 //     >= 0 receives particlesPerBlock particles at position + h * U[0, 1]^3 with the emitter's velocity.
 //
 // B200 design: the band distances are one CTA per triangle over its index box, min-combined with 64-bit
-// atomicMin on the bits of the non-negative distances (the same minimum as the reference's sequential loop); the
-// signs are one thread per node summing the winding terms of all triangles.  The distance arithmetic follows the
+// atomicMin on the bits of the non-negative distances (the same minimum as the reference's sequential loop).  The
+// signs of a closed mesh come from the grid rows: away from the surface its winding sum is 2 pi times an integer that
+// changes only where a row crosses a triangle, so one pass over the triangles records the crossings and one over the
+// rows adds them up; nodes whose row passes within rounding of an edge, or whose crossing lies within 1e-6 cells of a
+// node, sum the winding terms of all triangles, a warp per node.  Of an open mesh every node does, one thread per node
+// (fe_mesh_to_sdf of 1280 triangles on 96^3 nodes, copies included: 13.2 ms that way, 1.6 ms by rows).  The distance arithmetic follows the
 // reference's expressions in FP64 with round-to-nearest intrinsics, so distances are bit-identical; the sign test
 // sums CUDA's atan2, whose last bits can differ from the host library's, which decides nothing unless a node lies
 // within ~1e-12 of the 2 pi - 0.001 threshold (points on the surface sum to pi, points inside to 2 pi).  Seeding
@@ -59,10 +63,201 @@ __global__ void __launch_bounds__(256) k_mesh_band(MeshView m, NodeGrid g, unsig
     }
 }
 
-// TriangleMesh::IsInside at every node, then the signed value: -d inside, d outside.
-__global__ void __launch_bounds__(256) k_mesh_sign(MeshView m, NodeGrid g, const unsigned long long* __restrict__ bits,
-                                                   double* __restrict__ sdf)
+// Whether the mesh is closed: every edge, as a pair of vertex positions, is used as often in one direction as in the
+// other.  Each use adds a hash of the undirected edge, with its direction as the sign, to two 64-bit sums, which are
+// zero for a closed mesh (and for an open one with probability 2^-128).  Then the solid angles of its triangles sum to
+// an integer times 4 pi at every point off the surface.  state: the two sums, then non-zero if a coordinate is not
+// finite.
+__device__ __forceinline__ unsigned long long mix64(unsigned long long z)
 {
+    z += 0x9E3779B97F4A7C15ull;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return z ^ (z >> 31);
+}
+__device__ __forceinline__ unsigned long long hash_point(const double p[3], unsigned long long seed)
+{
+    unsigned long long h = seed;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) h = mix64(h ^ (unsigned long long)__double_as_longlong(p[a] + 0.0));  // -0 as 0
+    return h;
+}
+__device__ __forceinline__ int compare_points(const double p[3], const double q[3])
+{
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (p[a] < q[a]) return -1;
+        if (p[a] > q[a]) return 1;
+    }
+    return 0;
+}
+__global__ void __launch_bounds__(256) k_mesh_closed(MeshView m, unsigned long long* __restrict__ state)
+{
+    unsigned long long s0 = 0, s1 = 0;
+    bool bad = false;
+    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < m.nt; t += (uint64_t)gridDim.x * blockDim.x) {
+        double p[3][3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) load_vertex(m, m.T[4 * t + k], p[k]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) bad |= !isfinite(p[k][a]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double* u = p[k];
+            const double* v = p[(k + 1) % 3];
+            const int c = compare_points(u, v);
+            if (c == 0) continue;  // no edge
+            const double* lo = c < 0 ? u : v;
+            const double* hi = c < 0 ? v : u;
+            const unsigned long long h0 = mix64(hash_point(lo, 1) + 3 * hash_point(hi, 2));
+            const unsigned long long h1 = mix64(hash_point(lo, 5) ^ (hash_point(hi, 7) << 1 | 1));
+            s0 += c < 0 ? h0 : 0ull - h0;
+            s1 += c < 0 ? h1 : 0ull - h1;
+        }
+    }
+    if (s0) atomicAdd(state, s0);
+    if (s1) atomicAdd(state + 1, s1);
+    if (bad) atomicOr(state + 2, 1ull);
+}
+__device__ __forceinline__ bool mesh_closed(const unsigned long long* state)
+{
+    return (state[0] | state[1] | state[2]) == 0ull;
+}
+
+// Crossings of the grid rows along x with the triangles of a closed mesh, a warp per triangle, a lane per row.  cross[c]:
+// .x the change of the winding number (half the winding sum over pi) from node c - 1 to c of the row -- at the first
+// node, from far to the left --, .y non-zero where the node is to sum the winding terms itself.  Going in +x through a
+// triangle whose projection on (y, z) is positively oriented leaves the side its normal points away from: -1.
+// The projected point is in the triangle when its three edge functions have one sign; `tol` bounds their rounding.
+__global__ void __launch_bounds__(256) k_mesh_cross(MeshView m, NodeGrid g, const unsigned long long* __restrict__ state,
+                                                    int2* __restrict__ cross)
+{
+    if (!mesh_closed(state)) return;
+    const int lane = threadIdx.x & 31;
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    for (uint64_t t = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); t < m.nt; t += warps) {
+        double A[3], B[3], C[3], lo[3], hi[3], big = 0.0;
+        load_vertex(m, m.T[4 * t], A);
+        load_vertex(m, m.T[4 * t + 1], B);
+        load_vertex(m, m.T[4 * t + 2], C);
+        int first[3], last[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = fmin(A[a], fmin(B[a], C[a]));
+            hi[a] = fmax(A[a], fmax(B[a], C[a]));
+            big = fmax(big, fmax(fabs(lo[a]), fabs(hi[a])) + fabs(g.o[a]));
+            // nodes at or between the ends, with a margin for the rounding of the positions
+            const double f0 = (lo[a] - g.o[a]) / g.h[a], f1 = (hi[a] - g.o[a]) / g.h[a];
+            first[a] = (int)fmax(fmin(ceil(f0 - 1e-6), 2e9), -2e9);
+            last[a] = (int)fmax(fmin(floor(f1 + 1e-6), 2e9), -2e9);
+        }
+        const int j0 = max(first[1], 0), j1 = min(last[1], g.n[1] - 1), k0 = max(first[2], 0), k1 = min(last[2], g.n[2] - 1);
+        if (j1 < j0 || k1 < k0) continue;
+        const double span = (hi[1] - lo[1]) + (hi[2] - lo[2]);
+        const double tol = 1e-12 * span * (big + (g.n[1] - 1) * g.h[1] + (g.n[2] - 1) * g.h[2]);
+        const int64_t rows = (int64_t)(j1 - j0 + 1) * (k1 - k0 + 1);
+        for (int64_t q = lane; q < rows; q += 32) {
+            const int j = j0 + (int)(q % (j1 - j0 + 1)), k = k0 + (int)(q / (j1 - j0 + 1));
+            const double y = grid_pos(g, 1, j), z = grid_pos(g, 2, k);
+            auto edge = [&](const double* u, const double* v) { return (v[1] - u[1]) * (z - u[2]) - (v[2] - u[2]) * (y - u[1]); };
+            const double ab = edge(A, B), bc = edge(B, C), ca = edge(C, A);
+            const double emin = fmin(ab, fmin(bc, ca)), emax = fmax(ab, fmax(bc, ca));
+            if (emin < -tol && emax > tol) continue;  // clearly outside
+            const double area = ab + bc + ca;
+            int from = 1, to = 0;  // nodes that sum for themselves
+            if (emin > tol || emax < -tol) {
+                const double f = ((bc * A[0] + ca * B[0] + ab * C[0]) / area - g.o[0]) / g.h[0];
+                const double slack = 1e-6 + 4.0 * tol / fabs(area) * (hi[0] - lo[0]) / g.h[0];
+                const double r = rint(f);
+                if (slack > 0.25) {
+                    from = first[0] - 2;
+                    to = last[0] + 2;
+                } else if (fabs(f - r) <= slack) {
+                    from = (int)fmax(fmin(r, 2e9), -2e9);
+                    to = from + 1;
+                } else {
+                    const double at = fmax(ceil(f), 0.0);  // the first node after the crossing
+                    if (at <= g.n[0] - 1) atomicAdd(&cross[idx3((int)at, j, k, g.n[0], g.n[1])].x, area < 0.0 ? 1 : -1);
+                }
+            } else {  // within rounding of an edge
+                from = first[0] - 2;
+                to = last[0] + 2;
+            }
+            if (from <= to) {
+                from = max(from, 0);
+                to = min(max(to, 0), g.n[0] - 1);  // left of the grid: the row's first node
+                for (int i = from; i <= to; ++i) cross[idx3(i, j, k, g.n[0], g.n[1])].y = 1;
+            }
+        }
+    }
+}
+
+// TriangleMesh::IsInside at every node, then the signed value: -d inside, d outside.  k_mesh_rows: a closed mesh, a
+// warp per row, from the crossings (which share memory with the result: each lane reads its node's before it writes
+// it).  A node that sums for itself fixes the winding number for the nodes after it, unless it lies on the surface;
+// then the next one sums too.  k_mesh_sign: an open mesh, a thread per node.
+__global__ void __launch_bounds__(256) k_mesh_rows(MeshView m, NodeGrid g, const unsigned long long* __restrict__ state,
+                                                   const unsigned long long* __restrict__ bits, double* sdf)
+{
+    if (!mesh_closed(state)) return;
+    const double pi = 3.14159265358979323846;
+    const double two_pi_tol = ds(dm(2.0, pi), 0.001);
+    const int2* cross = reinterpret_cast<const int2*>(sdf);
+    const int lane = threadIdx.x & 31;
+    const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5), rows = (size_t)g.n[1] * g.n[2];
+    for (size_t row = blockIdx.x * (size_t)(blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
+        const int j = (int)(row % g.n[1]), k = (int)(row / g.n[1]);
+        int w = 0;
+        bool known = true;
+        for (int i0 = 0; i0 < g.n[0]; i0 += 32) {
+            const int i = i0 + lane, count = min(32, g.n[0] - i0);
+            const size_t c = idx3(i, j, k, g.n[0], g.n[1]);
+            const int2 x = lane < count ? cross[c] : make_int2(0, 0);
+            const unsigned own = __ballot_sync(0xffffffffu, x.y != 0);
+            bool inside = false;
+            if (known && own == 0u) {
+                int s = x.x;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int up = __shfl_up_sync(0xffffffffu, s, o);
+                    if (lane >= o) s += up;
+                }
+                inside = w + s != 0;
+                w += __shfl_sync(0xffffffffu, s, 31);
+            } else {
+                for (int q = 0; q < count; ++q) {
+                    const int step = __shfl_sync(0xffffffffu, x.x, q);
+                    bool in;
+                    if (!known || ((own >> q) & 1u)) {
+                        const double pt[3] = {grid_pos(g, 0, i0 + q), grid_pos(g, 1, j), grid_pos(g, 2, k)};
+                        double sum = winding_sum(m, pt, (uint64_t)lane, 32);
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) sum = da(sum, __shfl_xor_sync(0xffffffffu, sum, o));
+                        in = fabs(sum) >= two_pi_tol;
+                        const double turns = sum / (2.0 * pi);
+                        w = (int)rint(turns);
+                        known = fabs(turns - rint(turns)) < 1e-4;
+                    } else {
+                        w += step;
+                        in = w != 0;
+                    }
+                    if (lane == q) inside = in;
+                }
+            }
+            if (lane < count) {
+                const double d = __longlong_as_double((long long)bits[c]);
+                sdf[c] = inside ? dm(d, -1.0) : d;
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) k_mesh_sign(MeshView m, NodeGrid g, const unsigned long long* __restrict__ state,
+                                                   const unsigned long long* __restrict__ bits, double* __restrict__ sdf)
+{
+    if (m.nt && mesh_closed(state)) return;
     const double two_pi_tol = ds(dm(2.0, 3.14159265358979323846), 0.001);
     const size_t nc = (size_t)g.n[0] * g.n[1] * g.n[2];
     for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < nc; c += (size_t)gridDim.x * blockDim.x) {
@@ -186,7 +381,7 @@ NodeGrid node_grid(const int n[3], const double o[3], const double h[3])
 
 cudaError_t launch_mesh_to_sdf(const double* V, uint64_t nv, const int64_t* T, uint64_t nt, const int n[3],
                                const double o[3], const double h[3], unsigned long long* scratch, double* sdf,
-                               cudaStream_t st)
+                               unsigned long long* state, cudaStream_t st)
 {
     const NodeGrid g = node_grid(n, o, h);
     const size_t nc = (size_t)n[0] * n[1] * n[2];
@@ -202,7 +397,19 @@ cudaError_t launch_mesh_to_sdf(const double* V, uint64_t nv, const int64_t* T, u
         count_launch();
     }
     if (nv == 0) m.nt = 0;  // no vertices: no distances and no triangle to wind around (the fill stays positive)
-    k_mesh_sign<<<(unsigned)std::min<size_t>((nc + 255) / 256, 148 * 32), 256, 0, st>>>(m, g, scratch, sdf);
+    if (m.nt > 0) {
+        // the closed path's kernels and the open path's look at the sums and leave what is not theirs
+        cudaError_t e = cudaMemsetAsync(state, 0, kMeshStateWords * sizeof(unsigned long long), st);
+        if (e != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(sdf, 0, nc * sizeof(double), st)) != cudaSuccess) return e;
+        k_mesh_closed<<<(unsigned)std::min<uint64_t>((nt + 255) / 256, 148 * 8), 256, 0, st>>>(m, state);
+        k_mesh_cross<<<(unsigned)std::min<uint64_t>((nt + 7) / 8, 148 * 8), 256, 0, st>>>(m, g, state,
+                                                                                         reinterpret_cast<int2*>(sdf));
+        k_mesh_rows<<<(unsigned)std::min<size_t>(((size_t)n[1] * n[2] + 7) / 8, 148 * 32), 256, 0, st>>>(m, g, state, scratch,
+                                                                                                       sdf);
+        count_launch(3);
+    }
+    k_mesh_sign<<<(unsigned)std::min<size_t>((nc + 255) / 256, 148 * 32), 256, 0, st>>>(m, g, state, scratch, sdf);
     count_launch();
     return cudaGetLastError();
 }

@@ -1709,9 +1709,10 @@ fe_status fe_mesh_to_sdf(const double* vertices, uint64_t n_vertices, const int6
     const int nn[3] = {n[0], n[1], n[2]};
     fe_status r = upload_mesh(vertices, n_vertices, triangles, n_triangles, device, st, list, &dV, &dT);
     cudaError_t e = cudaSuccess;
-    if (r == FE_OK) e = dalloc(list, &scratch, nc, device, st);
+    if (r == FE_OK) e = dalloc(list, &scratch, nc + kMeshStateWords, device, st);
     if (r == FE_OK && e == cudaSuccess) e = dalloc(list, &dsdf, nc, device, st);
-    if (r == FE_OK && e == cudaSuccess) e = launch_mesh_to_sdf(dV, n_vertices, dT, n_triangles, nn, origin, spacing, scratch, dsdf, st);
+    if (r == FE_OK && e == cudaSuccess) e = launch_mesh_to_sdf(dV, n_vertices, dT, n_triangles, nn, origin, spacing, scratch, dsdf,
+                                                             scratch + nc, st);
     if (r == FE_OK && e == cudaSuccess) e = cudaMemcpyAsync(sdf, dsdf, nc * sizeof(double), cudaMemcpyDefault, st);
     if (r == FE_OK && e == cudaSuccess) e = cudaStreamSynchronize(st);
     free_list(list, st);
@@ -1744,9 +1745,12 @@ fe_status fe_scene_init_from_mesh(fe_scene* s, const double* vertices, uint64_t 
     if (r == FE_OK) e = dalloc(list, &count, nc, s->device, st);
     if (r == FE_OK && e == cudaSuccess) e = dalloc(list, &offset, nc + 1, s->device, st);
     if (r == FE_OK && e == cudaSuccess) e = dalloc(list, &tmp, tmp_bytes, s->device, st);
+    unsigned long long* state = nullptr;
+    if (r == FE_OK && e == cudaSuccess) e = dalloc(list, &state, kMeshStateWords, s->device, st);
     // Mesh2SDF into Fluid3::sdf, then InitializeParticles on it
     if (r == FE_OK && e == cudaSuccess)
-        e = launch_mesh_to_sdf(dV, n_vertices, dT, n_triangles, n, b.sdf_origin, b.h, s->surf.node, s->surf.sdf, st);
+        e = launch_mesh_to_sdf(dV, n_vertices, dT, n_triangles, n, b.sdf_origin, b.h, s->surf.node, s->surf.sdf,
+                               state, st);
     if (r == FE_OK && e == cudaSuccess) {
         s->mesh_sdf = true;
         s->prev_valid = false;
@@ -1807,8 +1811,9 @@ fe_status fe_scene_add_volume_emitter(fe_scene* s, const double* vertices, uint6
     fe_status r = upload_mesh(vertices, n_vertices, triangles, n_triangles, s->device, st, list, &dV, &dT);
     unsigned long long* scratch = nullptr;
     cudaError_t e = cudaSuccess;
-    if (r == FE_OK) e = dalloc(list, &scratch, nc, s->device, st);
-    if (r == FE_OK && e == cudaSuccess) e = launch_mesh_to_sdf(dV, n_vertices, dT, n_triangles, e2.n, e2.o, e2.h, scratch, e2.sdf, st);
+    if (r == FE_OK) e = dalloc(list, &scratch, nc + kMeshStateWords, s->device, st);
+    if (r == FE_OK && e == cudaSuccess)
+        e = launch_mesh_to_sdf(dV, n_vertices, dT, n_triangles, e2.n, e2.o, e2.h, scratch, e2.sdf, scratch + nc, st);
     free_list(list, st);
     cudaStreamSynchronize(st);
     if (r == FE_OK && e != cudaSuccess) r = cuda_check(e, "emitter sdf");
@@ -1969,9 +1974,9 @@ fe_status fe_scene_add_mesh_collider(fe_scene* s, const double* vertices, uint64
     if (e == cudaSuccess) e = cudaMemcpyAsync(dN, normals, 3 * n_normals * sizeof(double), cudaMemcpyDefault, st);
     if (e == cudaSuccess) e = dalloc(allocs, &dsdf, cn, s->device, st);
     std::vector<void*> tmp_list;
-    if (e == cudaSuccess) e = dalloc(tmp_list, &scratch, cn, s->device, st);
+    if (e == cudaSuccess) e = dalloc(tmp_list, &scratch, cn + kMeshStateWords, s->device, st);
     // TriangleMeshCollider's constructor: Mesh2SDF of the mesh on its own grid
-    if (e == cudaSuccess) e = launch_mesh_to_sdf(dV, n_vertices, dT, n_triangles, c.n, c.o, c.h, scratch, dsdf, st);
+    if (e == cudaSuccess) e = launch_mesh_to_sdf(dV, n_vertices, dT, n_triangles, c.n, c.o, c.h, scratch, dsdf, scratch + cn, st);
     free_list(tmp_list, st);
     if (e != cudaSuccess) {
         free_list(allocs, st);

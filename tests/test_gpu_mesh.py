@@ -170,3 +170,31 @@ def test_advance_frame_emits_every_substep():
     assert nsub >= 1
     first = 2 * int(((esdf <= 0) & (fluid >= 0)).sum())
     assert first > 0 and g.num_particles() - np0 >= first
+
+
+def _rotated(V, seed):
+    q, _ = np.linalg.qr(np.random.default_rng(seed).standard_normal((3, 3)))
+    return (V - 0.5) @ q + 0.5
+
+
+def _sign_meshes():
+    """Closed meshes whose grid rows pass through vertices, edges and faces, nested and overlapping bodies, inverted
+    orientation, a triangle soup, a mesh around the whole grid; and open ones."""
+    S, TS = icosphere((0.5, 0.5, 0.5), 0.3, 1)
+    B, TB = box((0.25, 0.25, 0.25), (0.75, 0.75, 0.75))  # faces on node planes
+    both = lambda a, b: (np.concatenate([a[0], b[0]]), np.concatenate([a[1], b[1] + np.array([len(a[0])] * 3 + [0])]))
+    flip = lambda T: T[:, [0, 2, 1, 3]]
+    soup = (S[TS[:, :3]].reshape(-1, 3), np.concatenate([np.arange(3 * len(TS)).reshape(-1, 3), TS[:, 3:]], 1))
+    return [("sphere_at_nodes", (S, TS)), ("box_at_nodes", (B, TB)), ("box_rotated", (_rotated(B, 1), TB)),
+            ("inverted", (S, flip(TS))), ("cavity", both((B, TB), (icosphere((0.5, 0.5, 0.5), 0.2, 1)[0], flip(TS)))),
+            ("overlap", both((B, TB), (S + 0.21, TS))), ("soup", soup),
+            ("around", (icosphere((0.5, 0.5, 0.5), 3.0, 1)[0], TS)), ("beside", (S + np.array([-0.4, 0.0, 0.1]), TS)),
+            ("open", (S, TS[:-3])), ("flat", (B, TB[:2])), ("degenerate", (B, np.concatenate([TB, [[0, 0, 3, 0]]])))]
+
+
+@pytest.mark.parametrize("name,mesh", _sign_meshes(), ids=[m[0] for m in _sign_meshes()])
+@pytest.mark.parametrize("n,h", [((16, 16, 16), 1 / 16), ((33, 9, 20), 1 / 20), ((70, 3, 5), 1 / 16)])
+def test_mesh_sdf_signs(name, mesh, n, h):
+    V, T = mesh
+    g = fe.mesh_to_sdf(V, T, n, (0.0, 0.0, 0.0), (h, h, h))
+    assert np.array_equal(g, oracle.mesh_to_sdf(V, T, n, (0.0, 0.0, 0.0), (h, h, h)))
