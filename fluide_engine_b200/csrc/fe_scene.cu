@@ -20,6 +20,8 @@
 #include <tuple>
 #include <vector>
 
+#include <cuda.h>
+
 #include "fe_internal.cuh"
 #include "fe_seed.h"
 
@@ -56,7 +58,7 @@ void count_launch(uint64_t n)
 
 namespace {
 
-__global__ void k_set_particles(SceneView v, const float* pos, const float* vel, const float* C, uint64_t n)
+__global__ void k_set_particles(SceneView v, const float* pos, const float* vel, bool zero_c, uint64_t n)
 {
     uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -67,8 +69,23 @@ __global__ void k_set_particles(SceneView v, const float* pos, const float* vel,
     v.vy[i] = vel ? vel[3 * i + 1] : 0.f;
     v.vz[i] = vel ? vel[3 * i + 2] : 0.f;
     v.pid[i] = (uint32_t)i;
-    if (v.solver == FE_SOLVER_APIC)
-        for (int a = 0; a < 9; ++a) v.c[a][i] = C ? C[9 * i + a] : 0.f;
+    if (zero_c)
+        for (int a = 0; a < 9; ++a) v.c[a][i] = 0.f;
+}
+
+// The APIC matrices, 9 floats a particle, into the 9 arrays: a block's rows go through shared memory, so both sides are
+// read and written in whole lines (as nine strided 2D copies: 60 us each for 0.6 M particles).
+constexpr int kSetC = 256;
+__global__ void __launch_bounds__(kSetC) k_set_c(SceneView v, const float* __restrict__ C, uint64_t n)
+{
+    __shared__ float rows[9 * kSetC];
+    const uint64_t i0 = blockIdx.x * (uint64_t)kSetC;
+    const int count = (int)(n - i0 < (uint64_t)kSetC ? n - i0 : (uint64_t)kSetC);
+    for (int q = threadIdx.x; q < 9 * count; q += kSetC) rows[q] = C[9 * i0 + q];
+    __syncthreads();
+    if ((int)threadIdx.x < count)
+#pragma unroll
+        for (int a = 0; a < 9; ++a) v.c[a][i0 + threadIdx.x] = rows[9 * threadIdx.x + a];
 }
 
 __global__ void k_sorted_keys(SceneView v, uint32_t* out)
@@ -185,6 +202,39 @@ struct fe_scene {
 };
 
 namespace {
+
+// Whether a kernel on the scene's device can use the caller's array of `floats` floats in place: ordinary memory of that
+// device, aligned to its elements, and the whole array inside the allocation that p points into (an array that is not
+// goes to the copy, which reports it).
+bool on_device(const fe_scene* s, const void* p, uint64_t floats)
+{
+    if (!p || ((uintptr_t)p & 3u)) return false;
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (a.type != cudaMemoryTypeDevice || a.device != s->device) return false;
+    using GetAttr = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+    static const GetAttr get = []() -> GetAttr {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return (GetAttr)f;
+    }();
+    if (!get) return false;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    const CUdeviceptr d = (CUdeviceptr)(uintptr_t)p;
+    if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, d) != CUDA_SUCCESS ||
+        get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, d) != CUDA_SUCCESS)
+        return false;
+    return d - start + floats * sizeof(float) <= size;
+}
 
 SceneView view_of(const fe_scene* s, int parity)
 {
@@ -1280,21 +1330,27 @@ fe_status fe_scene_set_particles(fe_scene* s, const float* pos, const float* vel
     s->base.np = n;
     s->parity = 0;
     if (n) {
-        // staging holds 9 floats per particle: pos at [0, 3n), vel at [3n, 6n); C reuses it afterwards
+        // arrays of this device are read where they are; others go through the staging buffer, which holds 9 floats per
+        // particle: pos at [0, 3n), vel at [3n, 6n); C reuses it afterwards
         float* stp = s->staging;
-        FE_CUDA(cudaMemcpyAsync(stp, pos, n * 3 * sizeof(float), cudaMemcpyDefault, s->stream));
-        if (vel) FE_CUDA(cudaMemcpyAsync(stp + 3 * n, vel, n * 3 * sizeof(float), cudaMemcpyDefault, s->stream));
+        const bool here = on_device(s, pos, 3 * n) && (!vel || on_device(s, vel, 3 * n));
+        if (!here) {
+            FE_CUDA(cudaMemcpyAsync(stp, pos, n * 3 * sizeof(float), cudaMemcpyDefault, s->stream));
+            if (vel) FE_CUDA(cudaMemcpyAsync(stp + 3 * n, vel, n * 3 * sizeof(float), cudaMemcpyDefault, s->stream));
+        }
         SceneView v = view_of(s, 0);
-        k_set_particles<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(v, stp, vel ? stp + 3 * n : nullptr,
-                                                                          nullptr, n);
+        const bool apic = s->desc.solver == FE_SOLVER_APIC;
+        k_set_particles<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(
+            v, here ? pos : stp, vel ? (here ? vel : stp + 3 * n) : nullptr, apic && !C, n);
         count_launch();
         FE_CUDA(cudaGetLastError());
-        if (C && s->desc.solver == FE_SOLVER_APIC) {
-            // stream order: the copy below starts after k_set_particles consumed the staging buffer
-            FE_CUDA(cudaMemcpyAsync(stp, C, n * 9 * sizeof(float), cudaMemcpyDefault, s->stream));
-            for (int a = 0; a < 9; ++a)  // deinterleave: c[a][i] = C[9 i + a]
-                FE_CUDA(cudaMemcpy2DAsync(v.c[a], sizeof(float), stp + a, 9 * sizeof(float), sizeof(float), n,
-                                          cudaMemcpyDeviceToDevice, s->stream));
+        if (C && apic) {
+            const bool c_here = on_device(s, C, 9 * n);
+            // stream order: the copy starts after k_set_particles consumed the staging buffer
+            if (!c_here) FE_CUDA(cudaMemcpyAsync(stp, C, n * 9 * sizeof(float), cudaMemcpyDefault, s->stream));
+            k_set_c<<<(unsigned)((n + kSetC - 1) / kSetC), kSetC, 0, s->stream>>>(v, c_here ? C : stp, n);
+            count_launch();
+            FE_CUDA(cudaGetLastError());
         }
     }
     FE_CUDA(cudaStreamSynchronize(s->stream));
@@ -1350,15 +1406,19 @@ fe_status fe_scene_get_particles(fe_scene* s, float* pos, float* vel, float* C, 
     FE_CUDA(cudaSetDevice(s->device));
     SceneView v = view_of(s, s->parity);
     float* stp = s->staging;
-    const bool wantC = C && s->desc.solver == FE_SOLVER_APIC;
-    FE_CUDA(launch_scatter_out(v, pos ? stp : nullptr, vel ? stp + 3 * n : nullptr, nullptr, s->stream));
-    if (pos) FE_CUDA(cudaMemcpyAsync(pos, stp, n * 3 * sizeof(float), cudaMemcpyDefault, s->stream));
-    if (vel) FE_CUDA(cudaMemcpyAsync(vel, stp + 3 * n, n * 3 * sizeof(float), cudaMemcpyDefault, s->stream));
-    if (wantC) {
+    const bool apic = s->desc.solver == FE_SOLVER_APIC;
+    // destinations on this device are written where they are; others through the staging buffer (9 floats per particle)
+    const bool pos_here = on_device(s, pos, 3 * n), vel_here = on_device(s, vel, 3 * n), c_here = on_device(s, C, 9 * n);
+    const bool c_early = C && apic && c_here;
+    FE_CUDA(launch_scatter_out(v, pos ? (pos_here ? pos : stp) : nullptr, vel ? (vel_here ? vel : stp + 3 * n) : nullptr,
+                               c_early ? C : nullptr, s->stream));
+    if (pos && !pos_here) FE_CUDA(cudaMemcpyAsync(pos, stp, n * 3 * sizeof(float), cudaMemcpyDefault, s->stream));
+    if (vel && !vel_here) FE_CUDA(cudaMemcpyAsync(vel, stp + 3 * n, n * 3 * sizeof(float), cudaMemcpyDefault, s->stream));
+    if (C && apic && !c_here) {
         FE_CUDA(cudaStreamSynchronize(s->stream));
         FE_CUDA(launch_scatter_out(v, nullptr, nullptr, stp, s->stream));
         FE_CUDA(cudaMemcpyAsync(C, stp, n * 9 * sizeof(float), cudaMemcpyDefault, s->stream));
-    } else if (C) {
+    } else if (C && !apic) {
         std::vector<float> z(n * 9, 0.f);
         FE_CUDA(cudaMemcpyAsync(C, z.data(), n * 9 * sizeof(float), cudaMemcpyDefault, s->stream));
         FE_CUDA(cudaStreamSynchronize(s->stream));
