@@ -265,7 +265,8 @@ cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t n, uint32_t* out,
                                   cudaStream_t st);
 cudaError_t launch_gather(const SceneView& v, const SceneView& dst, cudaStream_t st);
 cudaError_t launch_p2g(const SceneView& v, cudaStream_t st);
-cudaError_t launch_mark(const SceneView& v, cudaStream_t st);
+// cells_current: the cell starts are those of the particles' present positions (no move since the sort).
+cudaError_t launch_mark(const SceneView& v, bool cells_current, cudaStream_t st);
 cudaError_t launch_fluid_sdf(const SceneView& v, double* out, cudaStream_t st);
 // Distance bits of the band SDF per node by a particle scatter, then the diffusion face markers (fe_mark.cu).
 cudaError_t launch_face_fluid_marks(const SceneView& v, const DiffWork& d, cudaStream_t st);
@@ -524,6 +525,8 @@ G2PArgs g2p_args(const SceneView& v, double dt);
 struct MarkConst {
     double R2, rin2, crit_eps, inv_bucket;
     int two;
+    int fp32;             // FP32 distances decide all but the close cases:
+    float near2, far2;    // squared FP32 distances below near2 are within r, above far2 outside
 };
 
 constexpr int kBatchClearRanges = 8;

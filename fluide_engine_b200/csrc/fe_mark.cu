@@ -78,10 +78,8 @@ __device__ __forceinline__ void mark_node(const SceneView& v, const MarkConst& m
 // The common case, every axis' node window holding at most two nodes (cubic cells: 2r = 1.7 h): the 2 x 2 x 2
 // candidates are tested without loops, every table load issued first and each node's test predicated, so the
 // lanes of a warp stay converged.  Same nodes, same FP64 expressions and bucket tests as mark_body's loops.
-__device__ __forceinline__ void mark_body2(const SceneView& v, const MarkConst& mc, uint32_t blk)
+__device__ __forceinline__ void mark_particle2(const SceneView& v, const MarkConst& mc, uint64_t p)
 {
-    const uint64_t p = blk * (uint64_t)blockDim.x + threadIdx.x;
-    if (p >= v.np) return;
     const double X[3] = {(double)v.px[p], (double)v.py[p], (double)v.pz[p]};
     const int n[3] = {v.g.nx, v.g.ny, v.g.nz};
     int node[3][2];
@@ -111,6 +109,132 @@ __device__ __forceinline__ void mark_body2(const SceneView& v, const MarkConst& 
                 if (ok[2][sk] && ok[1][sj] && ok[0][si])
                     mark_node(v, mc, dist2_ref(X[0], X[1], X[2], q[0][si], q[1][sj], q[2][sk]), node[0][si],
                               node[1][sj], node[2][sk]);
+}
+
+// The same candidates in FP32: nodes base + (0|1, 0|1, 0|1) with squared distances d2[0][.] + d2[1][.] + d2[2][.].  A node
+// further inside r than the FP32 distance can be wrong is marked, one further outside is not; a particle with a node in
+// between (about one in 10^4), or too far from the grid, takes the exact test, which also lists the critical cells.  The
+// buckets need no test for a node inside r by that much: its search visits all of them.  near: bit a + 3 b + 9 c of the
+// nodes that are marked.  Returns false when the particle needs the exact test.
+__device__ __forceinline__ bool near_nodes(const SceneView& v, const MarkConst& mc, const float X[3], int base[3],
+                                           uint32_t& near)
+{
+    const int n[3] = {v.g.nx, v.g.ny, v.g.nz};
+    float d2[3][2];
+    bool in[3][2];
+    bool fine = mc.fp32 != 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float t = (X[a] - v.originf[a]) * v.inv_hf[a] - 0.5f;  // in cells from the first node
+        const float fl = floorf(t);
+        fine = fine && fabsf(t) < 1e6f;
+        base[a] = (int)fl;
+        const float lo = (t - fl) * v.hf[a], hi = (1.f - (t - fl)) * v.hf[a];
+        d2[a][0] = lo * lo;
+        d2[a][1] = hi * hi;
+        in[a][0] = (unsigned)base[a] < (unsigned)n[a];
+        in[a][1] = (unsigned)(base[a] + 1) < (unsigned)n[a];
+    }
+    near = 0;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        const int a = t & 1, b = (t >> 1) & 1, c = t >> 2;
+        const float d = d2[0][a] + d2[1][b] + d2[2][c];
+        const bool inside = in[0][a] && in[1][b] && in[2][c];
+        if (inside && d < mc.near2) near |= 1u << (a + 3 * b + 9 * c);
+        fine = fine && !(inside && d >= mc.near2 && d <= mc.far2);
+    }
+    return fine;
+}
+
+// One thread per particle (any order of the particles): 75 us at 128^3, bound by the byte stores; 100.7 with FP64 tests
+// of all 8 nodes.
+__device__ __forceinline__ void mark_particle(const SceneView& v, const MarkConst& mc, uint64_t p)
+{
+    const float X[3] = {v.px[p], v.py[p], v.pz[p]};
+    int base[3];
+    uint32_t near;
+    if (!near_nodes(v, mc, X, base, near)) {
+        mark_particle2(v, mc, p);
+        return;
+    }
+    const int64_t c0 = (int64_t)base[0] + (int64_t)v.g.nx * ((int64_t)base[1] + (int64_t)v.g.ny * (int64_t)base[2]);
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        const int a = t & 1, b = (t >> 1) & 1, c = t >> 2;
+        if ((near >> (a + 3 * b + 9 * c)) & 1u)
+            v.marks[c0 + a + (int64_t)v.g.nx * ((int64_t)b + (int64_t)v.g.ny * (int64_t)c)] = FE_CELL_FLUID;
+    }
+}
+__device__ __forceinline__ void mark_body2(const SceneView& v, const MarkConst& mc, uint32_t blk)
+{
+    const uint64_t p = blk * (uint64_t)blockDim.x + threadIdx.x;
+    if (p < v.np) mark_particle(v, mc, p);
+}
+
+// Many particles, sorted by their cells, in two passes, because nearly every cell that holds particles is marked by its
+// own: a particle is in reach of its cell's centre unless it sits in a corner, and stores of marks are what the pass
+// above is bound by.
+//   own    a thread per particle tests its own cell's node alone
+//   near   a block per 8^3-cell tile: the cells with an unmarked node among the 27 around them test all their particles
+//          against all their nodes, 8 lanes a cell; the others are done without reading a particle
+// A node that is marked needs no further test: one particle in reach decides it, and on grids with inexact cell-centre
+// samples a mark set from within crit_eps of r is listed when it is set, while one set from further inside makes the
+// sample negative whatever else is near.
+__device__ __forceinline__ void mark_own_body(const SceneView& v, const MarkConst& mc, uint32_t blk)
+{
+    const uint64_t p = blk * (uint64_t)blockDim.x + threadIdx.x;
+    if (p >= v.np) return;
+    const float X[3] = {v.px[p], v.py[p], v.pz[p]};
+    const int n[3] = {v.g.nx, v.g.ny, v.g.nz};
+    int c[3];
+    float d2 = 0.f;
+    bool in = mc.fp32 != 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float t = (X[a] - v.originf[a]) * v.inv_hf[a];
+        const float fl = floorf(t);
+        c[a] = (int)fl;
+        in = in && t >= 0.f && t < (float)n[a];
+        const float d = (t - fl - 0.5f) * v.hf[a];
+        d2 += d * d;
+    }
+    // the FP32 fraction is within near2's margin of the exact one whichever cell the rounding puts the particle in
+    if (in && d2 < mc.near2) v.marks[idx3(c[0], c[1], c[2], n[0], n[1])] = FE_CELL_FLUID;
+}
+struct MarkShared {
+    uint8_t open[10 * 10 * 10];       // 1 where a node in the grid is not marked: the tile and one cell around it
+    uint16_t list[FE_TILE_CELLS];     // cells to test
+    int count;
+};
+__device__ __forceinline__ void mark_near_body(const SceneView& v, const MarkConst& mc, int tile, MarkShared& sh)
+{
+    const uint32_t first = (uint32_t)tile * FE_TILE_CELLS;
+    if (v.cell_start[first] == v.cell_start[first + FE_TILE_CELLS]) return;
+    const int x0 = tile % v.g.tnx * FE_TILE, y0 = (tile / v.g.tnx) % v.g.tny * FE_TILE, z0 = tile / (v.g.tnx * v.g.tny) * FE_TILE;
+    if (threadIdx.x == 0) sh.count = 0;
+    for (int q = (int)threadIdx.x; q < 1000; q += (int)blockDim.x) {
+        const int i = x0 - 1 + q % 10, j = y0 - 1 + (q / 10) % 10, k = z0 - 1 + q / 100;
+        const bool in = (unsigned)i < (unsigned)v.g.nx && (unsigned)j < (unsigned)v.g.ny && (unsigned)k < (unsigned)v.g.nz;
+        sh.open[q] = in && v.marks[idx3(i, j, k, v.g.nx, v.g.ny)] != FE_CELL_FLUID ? 1 : 0;
+    }
+    __syncthreads();
+    for (int t = (int)threadIdx.x; t < FE_TILE_CELLS; t += (int)blockDim.x) {
+        if (v.cell_start[first + t] == v.cell_start[first + t + 1]) continue;
+        const uint8_t* o = sh.open + (t & 7) + 10 * ((t >> 3) & 7) + 100 * (t >> 6);
+        unsigned any = 0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) any |= o[10 * j + 100 * k] | o[10 * j + 100 * k + 1] | o[10 * j + 100 * k + 2];
+        if (any) sh.list[atomicAdd(&sh.count, 1)] = (uint16_t)t;
+    }
+    __syncthreads();
+    const int n = sh.count;
+    for (int e = (int)(threadIdx.x >> 3); e < n; e += (int)(blockDim.x >> 3)) {
+        const uint32_t key = first + sh.list[e];
+        for (uint32_t p = v.cell_start[key] + (threadIdx.x & 7), pe = v.cell_start[key + 1]; p < pe; p += 8) mark_particle(v, mc, p);
+    }
 }
 
 __device__ __forceinline__ void mark_body(const SceneView& v, const MarkConst& mc, uint32_t blk)
@@ -211,6 +335,13 @@ __device__ __forceinline__ void mark_fixup_body(const SceneView& v, double R2, u
 }
 
 __global__ void k_mark_fixup(SceneView v, double R2, uint32_t cap) { mark_fixup_body(v, R2, cap, blockIdx.x, gridDim.x); }
+
+__global__ void __launch_bounds__(256) k_mark_own(SceneView v, MarkConst mc) { mark_own_body(v, mc, blockIdx.x); }
+__global__ void __launch_bounds__(256) k_mark_near(SceneView v, MarkConst mc)
+{
+    __shared__ MarkShared sh;
+    mark_near_body(v, mc, (int)blockIdx.x, sh);
+}
 
 // ---- flat multi-scene forms (BatchPlan, fe_internal.cuh); marks, crit flags and counts are cleared by
 // launch_multi_clear
@@ -381,10 +512,22 @@ MarkConst mark_constants(const SceneView& v)
     mc.two = 1;
     for (int a = 0; a < 3; ++a)  // window (t - rr, t + rr] with rr = r / h_a + 1e-6 holds at most ceil(2 rr) nodes
         if (!(v.radius * v.inv_h[a] + 1e-6 < 1.0 - 1e-9)) mc.two = 0;
+    // FP32 distances: x - origin, its product with 1 / h and the fraction are each rounded, in all less than 2^-24 times
+    // |origin| + 4 |size| per axis and a few 2^-24 of the distance; twice that and more is left to the exact test
+    double reach = 0.0;
+    for (int a = 0; a < 3; ++a) reach = std::max(reach, std::fabs(v.origin[a]) + 4.0 * v.size[a]);
+    const double delta = 4.0 * std::sqrt(3.0) * 6e-8 * reach + 1e-5 * v.radius;
+    mc.fp32 = delta < 0.1 * v.radius ? 1 : 0;
+    mc.near2 = std::nextafterf((float)((v.radius - delta) * (v.radius - delta)), 0.f);
+    mc.far2 = std::nextafterf((float)((v.radius + delta) * (v.radius + delta)), HUGE_VALF);
     return mc;
 }
 
-cudaError_t launch_mark(const SceneView& v, cudaStream_t st)
+// From this many particles on the two passes take less time than the one.  The marking stage with its clears and launches,
+// one pass against two: 0.5 M particles (64^3) 39 us against 43, 0.6 M (61x90x47) 51.5 against 52.5, 2 M (100^3) 73 against
+// 66, 4 M (128^3) 91 against 79; of the kernels alone 75 us against 50 at 128^3 and 1018 against 363 at 256^3 (32 M).
+constexpr uint64_t kMarkTwoPasses = 1ull << 19;
+cudaError_t launch_mark(const SceneView& v, bool cells_current, cudaStream_t st)
 {
     const size_t nc = (size_t)v.g.nx * v.g.ny * v.g.nz;
     cudaError_t e = cudaMemsetAsync(v.marks, FE_CELL_AIR, nc, st);
@@ -395,8 +538,15 @@ cudaError_t launch_mark(const SceneView& v, cudaStream_t st)
         if ((e = cudaMemsetAsync(v.crit_count, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
     }
     if (v.np > 0) {
-        k_mark<<<(unsigned)((v.np + 255) / 256), 256, 0, st>>>(v, mc);
-        count_launch();
+        const unsigned nb = (unsigned)((v.np + 255) / 256);
+        if (mc.two && cells_current && v.np >= kMarkTwoPasses) {
+            k_mark_own<<<nb, 256, 0, st>>>(v, mc);
+            k_mark_near<<<(unsigned)(v.g.tnx * v.g.tny * v.g.tnz), 256, 0, st>>>(v, mc);
+            count_launch(2);
+        } else {
+            k_mark<<<nb, 256, 0, st>>>(v, mc);
+            count_launch();
+        }
         if (v.any_inexact) {
             k_mark_fixup<<<148, 128, 0, st>>>(v, mc.R2, (uint32_t)nc);
             count_launch();

@@ -153,6 +153,8 @@ struct fe_scene {
     // true once a substep's sort has run since the particles were set: the other particle set then holds the
     // positions at the start of the last substep, from which the reference's Fluid3::sdf was built
     bool prev_valid = false;
+    // the cell starts of the last sort are those of the particles' present positions (nothing moved or added since)
+    bool cells_current = false;
     // Fluid3::sdf holds the mesh SDF of fe_scene_init_from_mesh (in surf.sdf) until the next substep
     bool mesh_sdf = false;
     // BuildCollider has run (at the start of some substep): until then the collider SDF is its initial 0
@@ -722,6 +724,7 @@ fe_status enqueue_steps(fe_scene* s, double dt, int first, int last, cudaStream_
             FE_CUDA(launch_gather(v, dst, st));
             s->parity ^= 1;
             s->prev_valid = true;
+            s->cells_current = true;
             s->mesh_sdf = false;
             s->collider_built = true;
             break;
@@ -732,7 +735,7 @@ fe_status enqueue_steps(fe_scene* s, double dt, int first, int last, cudaStream_
             break;
         case kStepMark:
             if (s->colliders.count > 0) FE_CUDA(launch_collider_marks(v, s->cw, s->surf.node, &s->collider_fluid_sdf, st));
-            else FE_CUDA(launch_mark(v, st));
+            else FE_CUDA(launch_mark(v, s->cells_current, st));
             break;
         case kStepPre:
             FE_CUDA(ensure_grid(s, 0, st));
@@ -803,6 +806,7 @@ fe_status enqueue_steps(fe_scene* s, double dt, int first, int last, cudaStream_
             break;
         case kStepG2p:
             FE_CUDA(ensure_grid(s, 0, st));
+            if (last >= kStepMove) s->cells_current = false;
             if (last >= kStepMove && s->colliders.count > 0) {
                 // the collision response needs the state between the transfer and the move: no fusion
                 FE_CUDA(launch_g2p(v, dt, true, false, st));
@@ -819,6 +823,7 @@ fe_status enqueue_steps(fe_scene* s, double dt, int first, int last, cudaStream_
             break;
         case kStepMove:
             FE_CUDA(ensure_grid(s, 0, st));
+            s->cells_current = false;
             if (s->colliders.count > 0) FE_CUDA(launch_collider_keep_start(v, s->cw, st));
             FE_CUDA(launch_g2p(v, dt, false, true, st));
             if (s->colliders.count > 0) FE_CUDA(launch_collider_resolve(v, s->colliders, s->cw, collide_move(v, dt), st));
@@ -1005,6 +1010,7 @@ fe_status run_substep(fe_scene* s, double dt, cudaEvent_t* ev)
     }
     s->parity ^= 1;  // the sort inside the first graph flipped the buffer sets
     s->prev_valid = true;
+    s->cells_current = false;
     s->mesh_sdf = false;
     s->collider_built = true;
     s->grid_cur = 0;
@@ -1356,6 +1362,7 @@ fe_status fe_scene_set_particles(fe_scene* s, const float* pos, const float* vel
     FE_CUDA(cudaStreamSynchronize(s->stream));
     s->have_particles = true;
     s->prev_valid = false;
+    s->cells_current = false;
     return FE_OK;
 }
 
@@ -1387,6 +1394,7 @@ fe_status fe_scene_reset(fe_scene* s)
     FE_CUDA(cudaStreamSynchronize(st));
     s->grid_cur = 0;
     s->prev_valid = false;
+    s->cells_current = false;
     s->mesh_sdf = false;
     s->collider_built = false;
     s->collider_fluid_sdf = nullptr;
@@ -1742,6 +1750,7 @@ fe_status append_counted(fe_scene* s, const int n[3], const double o[3], const d
     FE_CUDA(cudaStreamSynchronize(st));
     s->base.np = np + total;
     s->have_particles = true;
+    s->cells_current = false;
     drop_graphs(s);
     return FE_OK;
 }
@@ -2443,6 +2452,7 @@ fe_status fe_scene_restore(fe_scene* s, const fe_snapshot* sn)
     }
     FE_CUDA(cudaStreamSynchronize(st));
     s->prev_valid = sn->prev_valid && sn->prev;
+    s->cells_current = false;
     s->collider_built = sn->collider_built;
     s->last_substep_empty = sn->last_substep_empty;
     s->have_particles = sn->have_particles;
@@ -2830,6 +2840,7 @@ void batch_after_substep(fe_batch* b)
     for (fe_scene* s : b->scenes) {
         s->parity ^= 1;
         s->prev_valid = true;
+        s->cells_current = false;
         s->mesh_sdf = false;
         s->collider_built = true;
         s->grid_cur = 0;
