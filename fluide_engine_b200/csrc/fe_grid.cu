@@ -568,7 +568,7 @@ uint32_t batch_blocks(const SceneView& v, int kind)
     switch (kind) {
     case kBkClear: return 0;  // set by the plan builder from its clear ranges
     case kBkPart: return (uint32_t)((v.np + 255) / 256);
-    case kBkP2g: return v.np > 0 ? (uint32_t)(v.g.tnx * v.g.tny * v.g.tnz) : 0u;
+    case kBkP2g: return v.np > 0 ? p2g_blocks(v) : 0u;
     case kBkNormalize: return (uint32_t)((faces + 1023) / 1024);  // four faces per thread
     case kBkFaces: {
         const dim3 g = column_grid(v.g.nx, v.g.ny, v.g.nz);

@@ -72,6 +72,7 @@ struct SceneView {
     // the sort's scratch: key per particle; rank = a particle's atomic slot in its cell, then (after the sort) the
     // sorted order, slot -> particle; perm = the runs in arbitrary order; cell counts and starts per cell key
     uint32_t *key, *rank, *perm, *cell_count, *cell_start;
+    uint32_t* p2g_list;    // P2G: how many quarter tiles hold more than a few particles, then those
     // grid
     float *u, *v, *w;
     float *u2, *v2, *w2;
@@ -265,6 +266,7 @@ cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t n, uint32_t* out,
                                   cudaStream_t st);
 cudaError_t launch_gather(const SceneView& v, const SceneView& dst, cudaStream_t st);
 cudaError_t launch_p2g(const SceneView& v, cudaStream_t st);
+uint32_t p2g_blocks(const SceneView& v);
 // cells_current: the cell starts are those of the particles' present positions (no move since the sort).
 cudaError_t launch_mark(const SceneView& v, bool cells_current, cudaStream_t st);
 cudaError_t launch_fluid_sdf(const SceneView& v, double* out, cudaStream_t st);
@@ -501,7 +503,7 @@ enum BatchKind {
     kBkScan,       // 1024 threads, 4096 counts each
     kBkScanSums,   // 1024 threads, one block per scene
     kBkBigcell,    // 1024 threads, striding over the scene's long runs
-    kBkP2g,        // one 8^3 cell tile each
+    kBkP2g,        // 128 threads, a quarter of an 8^3 cell tile each
     kBkNormalize,  // 256 threads, one face each
     kBkFaces,      // 32 x 8 threads, face_grid
     kBkCells,      // 32 x 8 threads, cell_grid

@@ -7,31 +7,40 @@
 // weight > 0.  PIC and APIC clamp the face index with the CELL count, FLIP with the face count.  APIC
 // adds C_row . (x_face - x_clamped), the particle position clamped by h/2 on the two transverse axes.
 //
-// B200 design: one CTA per 8x8x8-cell tile and one thread per cell of it.  The tile's particles are one
+// B200 design: a block takes a quarter of an 8x8x8-cell tile, one thread per cell.  A tile's particles are one
 // contiguous run of the sorted arrays (fe_keys.h) and a cell's particles a contiguous piece of that run, so
-// each thread walks its own cell's particles and sums their contributions in registers.  With the domain origin
+// each thread walks its own cell's particles once and sums all three components in registers.  With the domain origin
 // at zero the faces a particle of cell (cx, cy, cz) touches lie in a window around the cell -- faces c and c + 1
-// along the component's own axis, c - 1 .. c + 1 along the two others (the clamps of GetBarycentric at the domain
-// walls excepted: those particles take the direct path below) -- so a thread's sums live in 18 slots per
-// component, (numerator, weight) per window face, plus a touched mask.  Only then does the
-// thread add its touched slots into the tile's 10x10x10 face box in shared memory: one shared atomic per
-// (cell, face) pair instead of one per (particle, face) pair, and the 32 lanes of an atomic instruction hit 32
-// different faces.  Cells with more than kCellCap particles (particles clamped onto a wall pile up in one
+// along the component's own axis, c - 1 .. c + 1 along the two others -- so a thread's sums live in 18 slots per
+// component, (numerator, weight) per window face in one register pair for the packed FMA, plus a touched mask.  The
+// block's cells are first put in order of their particle counts, so a warp's lanes walk about equally many.  Only
+// then do the threads add their slots into the 10x10x4 face box in shared memory, slot after slot with a barrier
+// between: a slot is another face for every cell, so the adds need no atomics (shared FP32 atomics are compare-and-swap
+// loops).  Cells with more than kCellCap particles (particles clamped onto a wall pile up in one
 // cell) hand the rest to a warp that spreads them over its lanes and combines the lanes' slots by shuffles.
-// The box is then flushed to global accumulators: box faces touched by the tile get one global red.add each,
-// so a face receives at most 8 global adds (one per neighbouring tile), never one per particle.  A second pass
+// The box is then flushed to global accumulators: box faces touched by the block get one global red.add each,
+// so a face receives a few global adds (one per neighbouring part), never one per particle.  A second pass
 // divides numerator by weight and, for FLIP, writes the snapshot (flip_simulator.cpp:107-118).  A particle
 // whose stencil leaves its cell's window (only possible for a domain origin away from zero, where the
 // reference's data origins ignore the origin) takes the direct path instead: shared atomics into the box per
 // face, or global adds for faces outside the box, so the kernel stays correct for every input.
+//
+// Bound by instruction issue and the latency of a walk at 3 blocks (APIC 2) per SM.  A whole tile per block with one walk
+// per component and atomic box adds against this, the stage with its clears and normalisation: 65 against 60 us at 32^3
+// FLIP, 100 against 83 at 64^3 PIC, 138 against 106 at 61x90x47 APIC, 342 against 231 at 128^3 FLIP (4 M particles; the
+// splat kernels alone 249 against 176), 489 against 390 at 128^3 APIC, 1616 against 1326 at 200^3 APIC.
+#include <algorithm>
+
 #include "fe_internal.cuh"
 
 namespace fe {
 namespace {
 
-constexpr int kBox = 10;
-constexpr int kBoxFaces = kBox * kBox * kBox;
-constexpr int kP2gThreads = FE_TILE_CELLS;  // one thread per cell of a tile
+// A block takes a quarter of a tile, two cell layers along z, one thread per cell.
+constexpr int kP2gLayers = 2, kP2gParts = FE_TILE / kP2gLayers;
+constexpr int kP2gThreads = FE_TILE * FE_TILE * kP2gLayers;
+constexpr int kBox = 10, kBoxZ = kP2gLayers + 2;  // faces of the part and one around it
+constexpr int kBoxFaces = kBox * kBox * kBoxZ;
 constexpr int kCellCap = 32;                // particles a thread sums for its own cell; the rest go to a warp
 
 // Per-component constants of the transfer (face-array sizes, the clamp sizes the reference passes to
@@ -98,7 +107,7 @@ __device__ __forceinline__ P2gParticle<SOLVER> load_particle(const SceneView& v,
 // The particle's 8 faces added one by one: into the box (shared atomics) or, outside it, into the global
 // accumulators.  Used for particles whose stencil leaves their cell's window.
 template <int SOLVER>
-__device__ void splat_direct(const SceneView& v, const P2gComp& k, const Stencil& s, const P2gParticle<SOLVER>& q,
+__device__ __forceinline__ void splat_direct(const SceneView& v, const P2gComp& k, const Stencil& s, const P2gParticle<SOLVER>& q,
                              int bx, int by, int bz, float* s_num, float* s_den, uint8_t* s_mk)
 {
     const float wx[2] = {1.f - s.fx, s.fx}, wy[2] = {1.f - s.fy, s.fy}, wz[2] = {1.f - s.fz, s.fz};
@@ -115,7 +124,7 @@ __device__ void splat_direct(const SceneView& v, const P2gComp& k, const Stencil
             val += q.cr[0] * (gx - q.pc[0]) + q.cr[1] * (gy - q.pc[1]) + q.cr[2] * (gz - q.pc[2]);
         }
         const int li = ii[a] - bx, lj = jj[b] - by, lk = kk[d] - bz;
-        if ((unsigned)li < kBox && (unsigned)lj < kBox && (unsigned)lk < kBox) {
+        if ((unsigned)li < kBox && (unsigned)lj < kBox && (unsigned)lk < kBoxZ) {
             const int l = li + kBox * (lj + kBox * lk);
             atomicAdd(&s_num[l], val * wgt);
             atomicAdd(&s_den[l], wgt);
@@ -320,29 +329,242 @@ __device__ __forceinline__ void crowded_component(const SceneView& v, uint32_t o
     if (lane == 0) flush_slots<SOLVER, C>(ox, oy, oz, num, den, mask, s_num, s_den, s_mk);
 }
 
-template <int SOLVER, int C>
-__device__ __forceinline__ void own_component(const SceneView& v, uint32_t pb, uint32_t pe, int lx, int ly, int lz,
-                                              int cx, int cy, int cz, int bx, int by, int bz, const float lo[3],
-                                              const float hi[3], float* s_num, float* s_den, uint8_t* s_mk)
+// One axis of a particle's stencils.  The grid staggered along the axis has its two faces at the cell's sides (own
+// weights); the two grids that are not share one index and fraction (their data origins and sizes along it are the
+// same), the lower or the upper two of the window's three faces.  own_ok / tr_ok: the faces lie in the window.
+struct P2gAxis {
+    int oi, ti;        // first face of either pair
+    float of, tf;      // fractions
+    float own[2], tr[3];
+    bool own_ok, tr_ok, upper;
+    bool last;         // the cell counts clamp the own pair of the last cell's particles to faces c - 1 and c, weights 0, 1
+};
+__device__ __forceinline__ P2gAxis p2g_axis(float x, float own_org, float tr_org, float ih, int own_size, int n, int c)
 {
-    float num[nslots<C>()], den[nslots<C>()];
-    uint32_t mask;
-    cell_component<SOLVER, C>(v, pb, pe, 1u, cx, cy, cz, bx, by, bz, lo, hi, num, den, mask, s_num, s_den, s_mk);
-    flush_slots<SOLVER, C>(lx, ly, lz, num, den, mask, s_num, s_den, s_mk);
+    P2gAxis a;
+    bary((x - own_org) * ih, own_size - 1, a.oi, a.of);
+    bary((x - tr_org) * ih, n - 1, a.ti, a.tf);
+    a.last = a.oi == c - 1 && a.of == 1.f;
+    a.own_ok = a.oi == c || a.last;
+    a.upper = a.ti == c;
+    a.tr_ok = a.upper || a.ti == c - 1;
+    a.own[0] = a.last ? 1.f : 1.f - a.of;
+    a.own[1] = a.last ? 0.f : a.of;
+    const float lo = 1.f - a.tf;
+    a.tr[0] = a.upper ? 0.f : lo;
+    a.tr[1] = a.upper ? lo : a.tf;
+    a.tr[2] = a.upper ? a.tf : 0.f;
+    return a;
+}
+
+// (numerator, weight) of a face in one 64-bit register pair: the packed FP32 FMA adds to both at once.
+using Sum2 = unsigned long long;
+__device__ __forceinline__ Sum2 pack2(float a, float b)
+{
+    Sum2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(Sum2 s)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(s));
+    return r;
+}
+__device__ __forceinline__ Sum2 fma2(Sum2 a, Sum2 b, Sum2 c)
+{
+    Sum2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Component C of one particle into the cell's slots from its axes' weights: the sums of splat_slots.
+template <int SOLVER, int C>
+__device__ __forceinline__ void add_slots(const SceneView& v, const P2gAxis (&ax)[3], const float org[3], float vc,
+                                          const float cr[3], const float pc[3], const int c[3], const int l[3],
+                                          Sum2 (&sum)[nslots<C>()], uint32_t& mask, uint8_t* s_mk)
+{
+    constexpr int W0 = win<C>(0), W1 = win<C>(1), W2 = win<C>(2);
+    const float* wx = C == 0 ? ax[0].own : ax[0].tr;
+    const float* wy = C == 1 ? ax[1].own : ax[1].tr;
+    const float* wz = C == 2 ? ax[2].own : ax[2].tr;
+    const int up[3] = {C != 0 && ax[0].upper ? 1 : 0, C != 1 && ax[1].upper ? 1 : 0, C != 2 && ax[2].upper ? 1 : 0};
+    if (ax[C].last) {  // face c only; face c - 1 is touched with weight 0, which the marks show
+        mask |= spread_mask<C>(C == 0 ? 1u : 3u, C == 1 ? 1u : 3u, C == 2 ? 1u : 3u) << (up[0] + W0 * (up[1] + W1 * up[2]));
+        const int f[3] = {l[0] + (C == 0 ? 0 : up[0]), l[1] + (C == 1 ? 0 : up[1]), l[2] + (C == 2 ? 0 : up[2])};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {  // the other axes' two faces each
+            const int g[3] = {f[0] + (C == 0 ? 0 : (q & 1)), f[1] + (C == 1 ? 0 : (C == 0 ? (q & 1) : (q >> 1))),
+                              f[2] + (C == 2 ? 0 : (q >> 1))};
+            s_mk[g[0] + kBox * (g[1] + kBox * g[2])] = 1;
+        }
+    } else {
+        mask |= regular_mask<C>() << (up[0] + W0 * (up[1] + W1 * up[2]));
+    }
+    float gx[W0], dy[W1], dz[W2];
+    if (SOLVER == FE_SOLVER_APIC) {
+#pragma unroll
+        for (int r = 0; r < W0; ++r) gx[r] = cr[0] * ((org[0] + v.hf[0] * (float)(c[0] + wlo<C>(0) + r)) - pc[0]);
+#pragma unroll
+        for (int r = 0; r < W1; ++r) dy[r] = (org[1] + v.hf[1] * (float)(c[1] + wlo<C>(1) + r)) - pc[1];
+#pragma unroll
+        for (int r = 0; r < W2; ++r) dz[r] = (org[2] + v.hf[2] * (float)(c[2] + wlo<C>(2) + r)) - pc[2];
+    }
+    Sum2 w2[W0];
+#pragma unroll
+    for (int r = 0; r < W0; ++r) w2[r] = pack2(wx[r], wx[r]);
+#pragma unroll
+    for (int c3 = 0; c3 < W2; ++c3)
+#pragma unroll
+        for (int b3 = 0; b3 < W1; ++b3) {
+            const float a = wy[b3] * wz[c3];
+            if (SOLVER == FE_SOLVER_APIC) {
+                const float val = vc + (cr[1] * dy[b3] + cr[2] * dz[c3]);
+#pragma unroll
+                for (int a3 = 0; a3 < W0; ++a3) {
+                    Sum2& s = sum[a3 + W0 * (b3 + W1 * c3)];
+                    s = fma2(w2[a3], pack2(a * (val + gx[a3]), a), s);
+                }
+            } else {
+                const Sum2 ta = pack2(a * vc, a);
+#pragma unroll
+                for (int a3 = 0; a3 < W0; ++a3) {
+                    Sum2& s = sum[a3 + W0 * (b3 + W1 * c3)];
+                    s = fma2(w2[a3], ta, s);
+                }
+            }
+        }
 }
 
 // The tile's face box in shared memory (declared by the kernels, so a kernel that runs several transfer kinds holds
 // one box, not one per kind).
-struct P2gShared {
+struct __align__(16) P2gShared {
     float num[3][kBoxFaces];
     float den[3][kBoxFaces];
     uint8_t mk[3][kBoxFaces];
-    uint16_t over[FE_TILE_CELLS];  // cells with more than kCellCap particles (tile-local index)
+    uint16_t over[kP2gThreads];    // cells with more than kCellCap particles (index in the part)
     int nover;
+    int bin[kCellCap + 1];
+    uint16_t order[kP2gThreads];
 };
+static_assert(kCellCap == 32, "one lane per count below the cap");
+
+// Slot t of the window is another face for every cell, so the block adds slot after slot with a barrier between instead of
+// atomically (shared FP32 atomics are compare-and-swap loops).
+template <int C>
+__device__ __forceinline__ void flush_slot(int t, const int l[3], Sum2 sum, uint32_t mask, P2gShared& sh)
+{
+    if ((mask >> t) & 1u) {
+        const int f = slot_box<C>(l[0], l[1], l[2], t);
+        const float2 s = unpack2(sum);
+        sh.num[C][f] += s.x;
+        sh.den[C][f] += s.y;
+        sh.mk[C][f] = 1;
+    }
+}
+
+// A component of a particle whose faces leave the window (a domain origin away from zero).
+template <int SOLVER, int C>
+__device__ __forceinline__ void add_direct(const SceneView& v, uint32_t p, int bx, int by, int bz, const float lo[3],
+                                        const float hi[3], float* s_num, float* s_den, uint8_t* s_mk)
+{
+    const P2gComp k = p2g_comp<SOLVER>(v, C);
+    const float x = __ldg(v.px + p), y = __ldg(v.py + p), z = __ldg(v.pz + p);
+    const Stencil s = stencil(x, y, z, k.org, v.inv_hf, k.csx, k.csy, k.csz);
+    splat_direct<SOLVER>(v, k, s, load_particle<SOLVER>(v, p, C, x, y, z, lo, hi), bx, by, bz, s_num, s_den, s_mk);
+}
+
+
+// The cell's particles [pb, pe), all three components in one walk: 108 sums in registers, a particle's position and
+// velocity read once and its six axis weights computed once (three walks, one per component: 1224 thread instructions a
+// particle at 64^3 FLIP).
+template <int SOLVER>
+__device__ __forceinline__ void own_cell(const SceneView& v, uint32_t pb, uint32_t pe, const int c[3], const int l[3],
+                                         int bx, int by, int bz, const float lo[3], const float hi[3], P2gShared& sh)
+{
+    const bool flip = SOLVER == FE_SOLVER_FLIP;
+    Sum2 s0[18], s1[18], s2[18];
+#pragma unroll
+    for (int t = 0; t < 18; ++t) s0[t] = s1[t] = s2[t] = 0ull;
+    uint32_t m0 = 0, m1 = 0, m2 = 0;
+    for (uint32_t p = pb; p < pe; ++p) {
+        const float X[3] = {__ldg(v.px + p), __ldg(v.py + p), __ldg(v.pz + p)};
+        const float V[3] = {__ldg(v.vx + p), __ldg(v.vy + p), __ldg(v.vz + p)};
+        float cr[9], q[3] = {0.f, 0.f, 0.f};
+        if (SOLVER == FE_SOLVER_APIC) {
+#pragma unroll
+            for (int k = 0; k < 9; ++k) cr[k] = __ldg(v.c[k] + p);
+            // Clamp(val, max, min) on the transverse axes (apic_simulator.cpp:55-57,68-70,81-83)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) q[a] = X[a] < lo[a] ? lo[a] : (X[a] > hi[a] ? hi[a] : X[a]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 9; ++k) cr[k] = 0.f;
+        }
+        const P2gAxis ax[3] = {p2g_axis(X[0], v.xo[0], v.yo[0], v.inv_hf[0], flip ? v.g.nx + 1 : v.g.nx, v.g.nx, c[0]),
+                               p2g_axis(X[1], v.yo[1], v.xo[1], v.inv_hf[1], flip ? v.g.ny + 1 : v.g.ny, v.g.ny, c[1]),
+                               p2g_axis(X[2], v.zo[2], v.xo[2], v.inv_hf[2], flip ? v.g.nz + 1 : v.g.nz, v.g.nz, c[2])};
+        const float pu[3] = {X[0], q[1], q[2]}, pv[3] = {q[0], X[1], q[2]}, pw[3] = {q[0], q[1], X[2]};
+        if (ax[0].own_ok && ax[1].tr_ok && ax[2].tr_ok) add_slots<SOLVER, 0>(v, ax, v.xo, V[0], cr, pu, c, l, s0, m0, sh.mk[0]);
+        else add_direct<SOLVER, 0>(v, p, bx, by, bz, lo, hi, sh.num[0], sh.den[0], sh.mk[0]);
+        if (ax[0].tr_ok && ax[1].own_ok && ax[2].tr_ok) add_slots<SOLVER, 1>(v, ax, v.yo, V[1], cr + 3, pv, c, l, s1, m1, sh.mk[1]);
+        else add_direct<SOLVER, 1>(v, p, bx, by, bz, lo, hi, sh.num[1], sh.den[1], sh.mk[1]);
+        if (ax[0].tr_ok && ax[1].tr_ok && ax[2].own_ok) add_slots<SOLVER, 2>(v, ax, v.zo, V[2], cr + 6, pw, c, l, s2, m2, sh.mk[2]);
+        else add_direct<SOLVER, 2>(v, p, bx, by, bz, lo, hi, sh.num[2], sh.den[2], sh.mk[2]);
+    }
+    __syncthreads();  // the direct adds above are atomic and go to the same box
+#pragma unroll
+    for (int t = 0; t < 18; ++t) {
+        flush_slot<0>(t, l, s0[t], m0, sh);
+        flush_slot<1>(t, l, s1[t], m1, sh);
+        flush_slot<2>(t, l, s2[t], m2, sh);
+        __syncthreads();
+    }
+}
+
+// Parts of at most kFewParticles particles (spray) add each particle's faces to the global accumulators: setting up and
+// flushing the box would cost more.  `first` of `step` threads.
+constexpr uint32_t kFewParticles = 32;
+template <int SOLVER>
+__device__ __forceinline__ void few_particles(const SceneView& v, uint32_t beg, uint32_t end, uint32_t first, uint32_t step)
+{
+    const float lo[3] = {v.originf[0] + 0.5f * v.hf[0], v.originf[1] + 0.5f * v.hf[1], v.originf[2] + 0.5f * v.hf[2]};
+    const float hi[3] = {v.originf[0] + v.sizef[0] - 0.5f * v.hf[0], v.originf[1] + v.sizef[1] - 0.5f * v.hf[1],
+                         v.originf[2] + v.sizef[2] - 0.5f * v.hf[2]};
+    for (uint32_t e = first; e < 3 * (end - beg); e += step) {
+        const uint32_t p = beg + e / 3;
+        const int c = (int)(e % 3);
+        const P2gComp k = p2g_comp<SOLVER>(v, c);
+        const float x = __ldg(v.px + p), y = __ldg(v.py + p), z = __ldg(v.pz + p);
+        const Stencil s = stencil(x, y, z, k.org, v.inv_hf, k.csx, k.csy, k.csz);
+        // a box that no face lies in: every face goes to the global accumulators
+        splat_direct<SOLVER>(v, k, s, load_particle<SOLVER>(v, p, c, x, y, z, lo, hi), 1 << 24, 1 << 24, 1 << 24, nullptr,
+                             nullptr, nullptr);
+    }
+}
+__device__ __forceinline__ uint32_t part_first_key(int part)
+{
+    return (uint32_t)(part / kP2gParts) * FE_TILE_CELLS + (uint32_t)(part % kP2gParts) * (uint32_t)kP2gThreads;
+}
+
+// A warp per part: parts of few particles are done here, at full occupancy; the others are listed for k_p2g, whose blocks
+// (168 registers a thread) would otherwise mostly start up for parts with nothing or little to do.
+template <int SOLVER>
+__global__ void __launch_bounds__(256) k_p2g_few(SceneView v, int parts)
+{
+    const int part = (int)(blockIdx.x * 8 + (threadIdx.x >> 5)), lane = (int)(threadIdx.x & 31);
+    if (part >= parts) return;
+    const uint32_t first = part_first_key(part);
+    const uint32_t beg = v.cell_start[first], end = v.cell_start[first + kP2gThreads];
+    if (end - beg > kFewParticles) {
+        if (lane == 0) v.p2g_list[1 + atomicAdd(v.p2g_list, 1u)] = (uint32_t)part;
+    } else {
+        few_particles<SOLVER>(v, beg, end, (uint32_t)lane, 32u);
+    }
+}
 
 template <int SOLVER>
-__device__ __forceinline__ void p2g_body(const SceneView& v, int tile, P2gShared& sh)
+__device__ __forceinline__ void p2g_body(const SceneView& v, int part, P2gShared& sh)
 {
     float (&s_num)[3][kBoxFaces] = sh.num;
     float (&s_den)[3][kBoxFaces] = sh.den;
@@ -350,41 +572,61 @@ __device__ __forceinline__ void p2g_body(const SceneView& v, int tile, P2gShared
     uint16_t* s_over = sh.over;
     int& s_nover = sh.nover;
 
+    const int tile = part / kP2gParts, layer = part % kP2gParts * kP2gLayers;
     const int tx = tile % v.g.tnx, ty = (tile / v.g.tnx) % v.g.tny, tz = tile / (v.g.tnx * v.g.tny);
-    const int bx = tx * FE_TILE - 1, by = ty * FE_TILE - 1, bz = tz * FE_TILE - 1;  // box origin (face index)
-    const uint32_t beg = v.cell_start[(uint32_t)tile * FE_TILE_CELLS];
-    const uint32_t end = v.cell_start[(uint32_t)(tile + 1) * FE_TILE_CELLS];
+    const int x0 = tx * FE_TILE, y0 = ty * FE_TILE, z0 = tz * FE_TILE + layer;
+    const int bx = x0 - 1, by = y0 - 1, bz = z0 - 1;  // box origin (face index)
+    const uint32_t first = part_first_key(part);
+    const uint32_t beg = v.cell_start[first], end = v.cell_start[first + kP2gThreads];
     if (beg == end) return;  // nothing to splat; accumulators were cleared by the caller
-
-    for (int t = threadIdx.x; t < 3 * kBoxFaces; t += blockDim.x) {
-        (&s_num[0][0])[t] = 0.f;
-        (&s_den[0][0])[t] = 0.f;
-        (&s_mk[0][0])[t] = 0;
-    }
-    if (threadIdx.x == 0) s_nover = 0;
-    __syncthreads();
-
     const float lo[3] = {v.originf[0] + 0.5f * v.hf[0], v.originf[1] + 0.5f * v.hf[1], v.originf[2] + 0.5f * v.hf[2]};
     const float hi[3] = {v.originf[0] + v.sizef[0] - 0.5f * v.hf[0], v.originf[1] + v.sizef[1] - 0.5f * v.hf[1],
                          v.originf[2] + v.sizef[2] - 0.5f * v.hf[2]};
-
-    // this thread's cell (tile-local index = key & 511 = threadIdx.x)
-    const int lx = threadIdx.x & 7, ly = (threadIdx.x >> 3) & 7, lz = threadIdx.x >> 6;
-    const int cx = tx * FE_TILE + lx, cy = ty * FE_TILE + ly, cz = tz * FE_TILE + lz;
-    uint32_t pb = 0, pe = 0;
-    if (cx < v.g.nx && cy < v.g.ny && cz < v.g.nz) {
-        const uint32_t key = (uint32_t)tile * FE_TILE_CELLS + threadIdx.x;
-        pb = v.cell_start[key];
-        pe = v.cell_start[key + 1];
+    if (end - beg <= kFewParticles) {  // (in a flat batch launch; k_p2g_few has done them otherwise)
+        few_particles<SOLVER>(v, beg, end, threadIdx.x, blockDim.x);
+        return;
     }
+
+    for (int t = threadIdx.x; t < 3 * kBoxFaces / 4; t += blockDim.x) {
+        reinterpret_cast<float4*>(&s_num[0][0])[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        reinterpret_cast<float4*>(&s_den[0][0])[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        reinterpret_cast<uint32_t*>(&s_mk[0][0])[t] = 0u;
+    }
+    if (threadIdx.x == 0) s_nover = 0;
+    if (threadIdx.x <= (unsigned)kCellCap) sh.bin[threadIdx.x] = 0;
+    __syncthreads();
+
+    // the part's cells in order of their particle counts, one per thread: a warp's lanes then walk about equally many
+    // (in cell order a warp went on until its fullest cell was done: 14 rounds for 8 particles a cell)
+    int cell = (int)threadIdx.x;
+    {
+        const uint32_t count = min(v.cell_start[first + cell + 1] - v.cell_start[first + cell], (uint32_t)kCellCap);
+        const int at = atomicAdd(&sh.bin[count], 1);
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            int x = sh.bin[threadIdx.x];
+            const int own = x;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if ((int)threadIdx.x >= o) x += y;
+            }
+            sh.bin[threadIdx.x] = x - own;
+            if (threadIdx.x == 31) sh.bin[kCellCap] = x;
+        }
+        __syncthreads();
+        sh.order[sh.bin[count] + at] = (uint16_t)cell;
+        __syncthreads();
+        cell = sh.order[threadIdx.x];
+    }
+    const int l[3] = {cell & 7, (cell >> 3) & 7, cell >> 6};
+    const int c[3] = {x0 + l[0], y0 + l[1], z0 + l[2]};
+    uint32_t pb = v.cell_start[first + cell], pe = v.cell_start[first + cell + 1];  // none in cells outside the grid
     if (pe - pb > (uint32_t)kCellCap) {
-        s_over[atomicAdd(&s_nover, 1)] = (uint16_t)threadIdx.x;
+        s_over[atomicAdd(&s_nover, 1)] = (uint16_t)cell;
         pe = pb + kCellCap;
     }
-    own_component<SOLVER, 0>(v, pb, pe, lx, ly, lz, cx, cy, cz, bx, by, bz, lo, hi, s_num[0], s_den[0], s_mk[0]);
-    own_component<SOLVER, 1>(v, pb, pe, lx, ly, lz, cx, cy, cz, bx, by, bz, lo, hi, s_num[1], s_den[1], s_mk[1]);
-    own_component<SOLVER, 2>(v, pb, pe, lx, ly, lz, cx, cy, cz, bx, by, bz, lo, hi, s_num[2], s_den[2], s_mk[2]);
-    __syncthreads();
+    own_cell<SOLVER>(v, pb, pe, c, l, bx, by, bz, lo, hi, sh);
 
     // crowded cells: a warp per cell, lanes stride over the particles past kCellCap
     const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -392,14 +634,12 @@ __device__ __forceinline__ void p2g_body(const SceneView& v, int tile, P2gShared
     for (int o = warp; o < nover; o += nwarps) {
         const int t = s_over[o];
         const int ox = t & 7, oy = (t >> 3) & 7, oz = t >> 6;
-        const int ocx = tx * FE_TILE + ox, ocy = ty * FE_TILE + oy, ocz = tz * FE_TILE + oz;
-        const uint32_t key = (uint32_t)tile * FE_TILE_CELLS + (uint32_t)t;
-        const uint32_t ob = v.cell_start[key] + kCellCap, oe = v.cell_start[key + 1];
-        crowded_component<SOLVER, 0>(v, ob, oe, ox, oy, oz, ocx, ocy, ocz, bx, by, bz, lo, hi, s_num[0], s_den[0],
+        const uint32_t ob = v.cell_start[first + (uint32_t)t] + kCellCap, oe = v.cell_start[first + (uint32_t)t + 1];
+        crowded_component<SOLVER, 0>(v, ob, oe, ox, oy, oz, x0 + ox, y0 + oy, z0 + oz, bx, by, bz, lo, hi, s_num[0], s_den[0],
                                      s_mk[0]);
-        crowded_component<SOLVER, 1>(v, ob, oe, ox, oy, oz, ocx, ocy, ocz, bx, by, bz, lo, hi, s_num[1], s_den[1],
+        crowded_component<SOLVER, 1>(v, ob, oe, ox, oy, oz, x0 + ox, y0 + oy, z0 + oz, bx, by, bz, lo, hi, s_num[1], s_den[1],
                                      s_mk[1]);
-        crowded_component<SOLVER, 2>(v, ob, oe, ox, oy, oz, ocx, ocy, ocz, bx, by, bz, lo, hi, s_num[2], s_den[2],
+        crowded_component<SOLVER, 2>(v, ob, oe, ox, oy, oz, x0 + ox, y0 + oy, z0 + oz, bx, by, bz, lo, hi, s_num[2], s_den[2],
                                      s_mk[2]);
     }
     __syncthreads();
@@ -421,10 +661,14 @@ __device__ __forceinline__ void p2g_body(const SceneView& v, int tile, P2gShared
 }
 
 template <int SOLVER>
-__global__ void __launch_bounds__(kP2gThreads, 1) k_p2g(SceneView v)
+__global__ void __launch_bounds__(kP2gThreads, SOLVER == FE_SOLVER_APIC ? 2 : 3) k_p2g(SceneView v)
 {
     __shared__ P2gShared sh;
-    p2g_body<SOLVER>(v, (int)blockIdx.x, sh);
+    const uint32_t n = v.p2g_list[0];
+    for (uint32_t e = blockIdx.x; e < n; e += gridDim.x) {
+        p2g_body<SOLVER>(v, (int)v.p2g_list[1 + e], sh);
+        __syncthreads();  // the next part clears the box
+    }
 }
 
 // u = num / weight where weight > 0 (pic_simulator.cpp:414-436); FLIP also snapshots the result.
@@ -468,7 +712,7 @@ __global__ void __launch_bounds__(256) k_p2g_normalize(SceneView v, size_t total
 
 // ---- flat multi-scene forms (BatchPlan, fe_internal.cuh): every scene's tiles in one launch, each block running
 // its scene's transfer kind
-__global__ void __launch_bounds__(kP2gThreads, 1) k_multi_p2g(const BatchPlan* __restrict__ plan)
+__global__ void __launch_bounds__(kP2gThreads, 2) k_multi_p2g(const BatchPlan* __restrict__ plan)
 {
     __shared__ P2gShared sh;
     __shared__ SceneView v;
@@ -505,6 +749,8 @@ cudaError_t launch_multi_p2g(const BatchLaunch& L, cudaStream_t st)
     return cudaGetLastError();
 }
 
+uint32_t p2g_blocks(const SceneView& v) { return (uint32_t)(v.g.tnx * v.g.tny * v.g.tnz) * kP2gParts; }
+
 cudaError_t launch_p2g(const SceneView& v, cudaStream_t st)
 {
     const size_t nu = (size_t)(v.g.nx + 1) * v.g.ny * v.g.nz, nvv = (size_t)v.g.nx * (v.g.ny + 1) * v.g.nz,
@@ -514,12 +760,23 @@ cudaError_t launch_p2g(const SceneView& v, cudaStream_t st)
     if ((e = cudaMemsetAsync(v.nu, 0, (nu + nvv + nww) * sizeof(float), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(v.du, 0, (nu + nvv + nww) * sizeof(float), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(v.mu, 0, nu + nvv + nww, st)) != cudaSuccess) return e;
-    const unsigned tiles = (unsigned)(v.g.tnx * v.g.tny * v.g.tnz);
     if (v.np > 0) {
-        if (v.solver == FE_SOLVER_PIC) k_p2g<FE_SOLVER_PIC><<<tiles, kP2gThreads, 0, st>>>(v);
-        else if (v.solver == FE_SOLVER_FLIP) k_p2g<FE_SOLVER_FLIP><<<tiles, kP2gThreads, 0, st>>>(v);
-        else k_p2g<FE_SOLVER_APIC><<<tiles, kP2gThreads, 0, st>>>(v);
-        count_launch();
+        const int parts = (int)p2g_blocks(v);
+        if ((e = cudaMemsetAsync(v.p2g_list, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
+        const unsigned few = (unsigned)((parts + 7) / 8);
+        // persistent blocks: as many as are resident at once (3 per SM, APIC 2)
+        const unsigned grid = (unsigned)std::min(parts, 148 * (v.solver == FE_SOLVER_APIC ? 2 : 3));
+        if (v.solver == FE_SOLVER_PIC) {
+            k_p2g_few<FE_SOLVER_PIC><<<few, 256, 0, st>>>(v, parts);
+            k_p2g<FE_SOLVER_PIC><<<grid, kP2gThreads, 0, st>>>(v);
+        } else if (v.solver == FE_SOLVER_FLIP) {
+            k_p2g_few<FE_SOLVER_FLIP><<<few, 256, 0, st>>>(v, parts);
+            k_p2g<FE_SOLVER_FLIP><<<grid, kP2gThreads, 0, st>>>(v);
+        } else {
+            k_p2g_few<FE_SOLVER_APIC><<<few, 256, 0, st>>>(v, parts);
+            k_p2g<FE_SOLVER_APIC><<<grid, kP2gThreads, 0, st>>>(v);
+        }
+        count_launch(2);
     }
     const size_t total = nu + nvv + nww;
     const unsigned nb = (unsigned)((total + 1023) / 1024);
