@@ -759,12 +759,12 @@ cudaError_t launch_collider_bc(const SceneView& v, const CollideWork& w, float* 
     return cudaGetLastError();
 }
 
-cudaError_t launch_collider_marks(const SceneView& v, const CollideWork& w, unsigned long long* node_scratch,
-                                  double** fluid_sdf, cudaStream_t st)
+cudaError_t launch_collider_marks(const SceneView& v, const NodeCells& cells, const CollideWork& w, double** fluid_sdf,
+                                  cudaStream_t st)
 {
     const int nx = v.g.nx, ny = v.g.ny, nz = v.g.nz;
     const size_t nc = (size_t)nx * ny * nz;
-    cudaError_t e = launch_node_sdf(v, node_scratch, w.sdf_a, st);  // BuildSignedDistanceField
+    cudaError_t e = launch_node_sdf(v, cells, w.sdf_a, st);  // BuildSignedDistanceField
     if (e != cudaSuccess) return e;
     double* in = w.sdf_a;
     double* out = w.sdf_b;

@@ -369,14 +369,14 @@ cudaError_t diffuse_prepare(DiffWork& d, int device)
     return cudaSuccess;
 }
 
-cudaError_t launch_diffuse(const SceneView& v, const DiffWork& d, const CgWork& w, float* u, float* vv, float* ww,
-                           double dt, double viscosity, cudaStream_t st)
+cudaError_t launch_diffuse(const SceneView& v, const NodeCells& cells, const DiffWork& d, const CgWork& w, float* u, float* vv,
+                           float* ww, double dt, double viscosity, cudaStream_t st)
 {
     const int nx = v.g.nx, ny = v.g.ny, nz = v.g.nz;
     if (d.blocks < 1 || d.blocks > 1023) return cudaErrorInitializationError;  // k_jacobi packs block counts in 10 bits
     cudaError_t e;
     if ((e = cudaMemsetAsync(d.count, 0, sizeof(unsigned), st)) != cudaSuccess) return e;
-    if ((e = launch_face_fluid_marks(v, d, st)) != cudaSuccess) return e;
+    if ((e = launch_face_fluid_marks(v, cells, d, st)) != cudaSuccess) return e;
     FaceArrays3 fa;
     fa.vel[0] = u;
     fa.vel[1] = vv;

@@ -245,7 +245,7 @@ __device__ __forceinline__ bool column_coord(int nx, int ny, int nz, Blk3 b, Fac
 // Viscosity (fe_diffuse.cu): buffers of the implicit diffusion solve, allocated when a scene's viscosity is > 0.
 // Face arrays are the three components concatenated (u | v | w) like the velocity buffers.
 struct DiffWork {
-    unsigned long long* node_dist;  // nx*ny*nz: bits of the smallest particle distance per SDF node (all ones: none)
+    double* node;                   // nx*ny*nz: the fluid's band SDF
     uint8_t* mark;                  // faces: FE_CELL_FLUID / FE_CELL_AIR (BackwardEulerDiffusionSolver::_fluidMarkers)
     unsigned long long* list;       // FLUID faces: (face << 9) | (wall << 8) | (component << 6) | FLUID-neighbour mask
     double* x[2];                   // faces: Jacobi iterates (only FLUID entries are used)
@@ -260,6 +260,8 @@ struct DiffWork {
 
 // Kernel launchers (one per .cu file).
 cudaError_t launch_sort(const SceneView& v, cudaStream_t st, void* scan_tmp, size_t scan_tmp_bytes);
+// The sort up to the cells' runs: v.cell_start, and in v.perm each cell's particles in arbitrary order.
+cudaError_t launch_group(const SceneView& v, cudaStream_t st, void* scan_tmp, size_t scan_tmp_bytes);
 size_t sort_scan_tmp_bytes(uint32_t n);
 // Exclusive prefix sum of n counts into out[0..n] (out[n] = total); tmp holds sort_scan_tmp_bytes(n).
 cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t n, uint32_t* out, void* tmp, size_t tmp_bytes,
@@ -270,11 +272,18 @@ uint32_t p2g_blocks(const SceneView& v);
 // cells_current: the cell starts are those of the particles' present positions (no move since the sort).
 cudaError_t launch_mark(const SceneView& v, bool cells_current, cudaStream_t st);
 cudaError_t launch_fluid_sdf(const SceneView& v, double* out, cudaStream_t st);
-// Distance bits of the band SDF per node by a particle scatter, then the diffusion face markers (fe_mark.cu).
-cudaError_t launch_face_fluid_marks(const SceneView& v, const DiffWork& d, cudaStream_t st);
-// The band SDF of v's particles at every node (BuildSignedDistanceField's values, FP64) by the same scatter;
-// node_scratch holds nx*ny*nz u64 (fe_mark.cu).
-cudaError_t launch_node_sdf(const SceneView& v, unsigned long long* node_scratch, double* sdf, cudaStream_t st);
+// v's particles by cell: where each cell's run starts (key_space + 1; null: not known) and the particle of each slot of the
+// runs (null: the slot's own, v is sorted).
+struct NodeCells {
+    const uint32_t* start;
+    const uint32_t* order;
+};
+// The band SDF of v's particles at every node (BuildSignedDistanceField's values, FP64; fe_mark.cu): gathered from the cells
+// where they are known, scattered by the particles otherwise.
+cudaError_t launch_node_sdf(const SceneView& v, const NodeCells& cells, double* sdf, cudaStream_t st);
+bool node_sdf_uses_cells(const SceneView& v);
+// The band SDF into d.node, then the diffusion face markers.
+cudaError_t launch_face_fluid_marks(const SceneView& v, const NodeCells& cells, const DiffWork& d, cudaStream_t st);
 cudaError_t launch_pre(const SceneView& v, double dt, cudaStream_t st);
 cudaError_t launch_post(const SceneView& v, cudaStream_t st);
 cudaError_t launch_rhs(const SceneView& v, cudaStream_t st);
@@ -451,8 +460,8 @@ cudaError_t launch_collider_face_lists(const SceneView& v, CollideWork& w, bool 
 cudaError_t launch_collider_bc(const SceneView& v, const CollideWork& w, float* const buf[3], cudaStream_t st);
 // Enclosed FLUID components (no AIR neighbour: a pure-Neumann block) lose the mean of their right-hand side.
 cudaError_t launch_collider_project_rhs(const SceneView& v, const CollideWork& w, int* err, cudaStream_t st);
-cudaError_t launch_collider_marks(const SceneView& v, const CollideWork& w, unsigned long long* node_scratch,
-                                  double** fluid_sdf, cudaStream_t st);
+cudaError_t launch_collider_marks(const SceneView& v, const NodeCells& cells, const CollideWork& w, double** fluid_sdf,
+                                  cudaStream_t st);
 cudaError_t launch_collider_keep_start(const SceneView& v, const CollideWork& w, cudaStream_t st);
 cudaError_t launch_collider_resolve(const SceneView& v, const CollideSet& cs, const CollideWork& w,
                                     const CollideMove& g, cudaStream_t st);
@@ -484,8 +493,8 @@ cudaError_t launch_forces(const SceneView& v, const ForceList& fl, float* u, flo
 
 // Viscosity (fe_diffuse.cu): ComputeDiffusion on the velocity buffers u, vv, ww (face markers, FLUID-face list,
 // persistent Jacobi solve, wall layers zeroed).  Uses the scene's solver barrier and error words (CgWork).
-cudaError_t launch_diffuse(const SceneView& v, const DiffWork& d, const CgWork& w, float* u, float* vv, float* ww,
-                           double dt, double viscosity, cudaStream_t st);
+cudaError_t launch_diffuse(const SceneView& v, const NodeCells& cells, const DiffWork& d, const CgWork& w, float* u, float* vv,
+                           float* ww, double dt, double viscosity, cudaStream_t st);
 cudaError_t diffuse_prepare(DiffWork& d, int device);
 
 // ------------------------------------------------------------------ flat multi-scene launches (batches)

@@ -384,7 +384,8 @@ __global__ void k_fluid_sdf(SceneView v, double R2, double* out)
 // (dx^2 + dy^2) + dz^2; a row whose dy^2 + dz^2 already exceeds (2r)^2 is skipped (rounding is monotonic, so the
 // full sum would exceed it too), and the bucket test runs once per axis.  Particles sorted by cell hit the same
 // nodes as their neighbours; a plain read of the current minimum first (it only decreases, so a stale value is
-// still an upper bound) skips most atomics.
+// still an upper bound) skips most atomics.  For particles whose cells are not known and bands wider than k_sdf_gather's
+// reach.
 __global__ void __launch_bounds__(256) k_sdf_scatter(SceneView v, unsigned long long* __restrict__ node, double R2)
 {
     uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -441,11 +442,278 @@ __device__ __forceinline__ double node_value(unsigned long long raw, double band
     return __dsub_rn(m, radius);
 }
 
-__global__ void k_node_values(const unsigned long long* __restrict__ node, size_t nc, double band, double radius,
-                              double* __restrict__ sdf)
+// In place: a node's distance bits become its value.
+__global__ void k_node_values(double* node, size_t nc, double band, double radius)
 {
     for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < nc; c += (size_t)gridDim.x * blockDim.x)
-        sdf[c] = node_value(node[c], band, radius);
+        node[c] = node_value((unsigned long long)__double_as_longlong(node[c]), band, radius);
+}
+
+// The same node values from particles that are grouped by cell, gathered per node: no atomics, and nearly every node
+// inside the fluid is decided by its own cell, because a particle nearer than half a cell is nearer than any of another
+// cell.  A block takes a tile's nodes.  Nodes whose own cell doesn't decide are listed, so that warps are full again, and
+// walk the occupied cells up to two away (the band is at most 2.5 cells wide, see node_reach), nearer rows first; a row or
+// cell is skipped when its nearest point is further away than the smallest distance so far.  The bucket test of the
+// reference's search is made for the nearest particle alone.  Where it fails (the nearest one doesn't count), or a cell holds
+// too many particles for one thread, a warp searches all cells with the test for each particle.  `order` (optional) gives
+// the particle of each slot of the cells' runs.
+//
+// Bound by the latency of the listed nodes' searches (a lone particle has some 80 nodes search for it).  Against the scatter
+// over particles below, which tests 64 nodes a particle and reads 21 of them: 4 M particles at 128^3 (FLIP dam with spray,
+// unsorted) 512 us against 208, and 50 for grouping them; 0.5 M sorted ones at 64^3 92 against 58.  With one walk over the
+// rows instead of the groups of bits 321 and 82, with a warp per listed node 630 and 160.
+//
+// The 125 cells around a node come in five groups, nearer ones first: the 27 that touch the node's cell, those two away along
+// x in the same rows, then the 16 rows around (6, 6 and 4 of 5 cells).  A thread collects a group's occupied cells as bits
+// and visits bit after bit, so that the lanes of a warp, whose nodes lie next to other cells, all have a cell to visit.
+constexpr int kNodeGroups = 5, kNodeCells = 125;
+struct NodeReach {
+    double near2[kNodeCells];         // squared distance from a node to the nearest point of the cell
+    double group2[kNodeGroups];       // the smallest of the group
+    uint32_t valid[kNodeGroups];      // cells that reach into the band
+    double own2;                      // squared distance up to which the node's own cell decides
+};
+__host__ __device__ constexpr int node_group_first(int w) { return w == 0 ? 0 : (w == 1 ? 27 : 45 + 30 * (w - 2)); }
+// Rows around a node, (dy + 2) + 5 (dz + 2): the 9 that touch its cell's row, then the 16 around, nearer ones first.
+__host__ __device__ constexpr int node_row(int r)
+{
+    constexpr int rows[25] = {12, 7, 11, 13, 17, 6, 8, 16, 18, 2, 10, 14, 22, 1, 3, 5, 9, 15, 19, 21, 23, 0, 4, 20, 24};
+    return rows[r];
+}
+// Offset of the cell of bit `bit` of group `w`.
+__host__ __device__ inline void node_cell(int w, int bit, int d[3])
+{
+    const int width = w == 0 ? 3 : (w == 1 ? 2 : 5);
+    const int row = node_row(w < 2 ? bit / width : 9 + 6 * (w - 2) + bit / width), x = bit % width;
+    d[0] = w == 0 ? x - 1 : (w == 1 ? 4 * x - 2 : x - 2);
+    d[1] = row % 5 - 2;
+    d[2] = row / 5 - 2;
+}
+
+// A block takes half a tile: 256 nodes, and the cells up to two around them.
+constexpr int kNodeLayers = FE_TILE / 2;
+constexpr int kNodeThreads = FE_TILE * FE_TILE * kNodeLayers;
+constexpr int kNodeHalo = FE_TILE + 4, kNodeHaloZ = kNodeLayers + 4;
+constexpr uint32_t kNodeLaneCap = 32;  // particles a thread tests for one cell; fuller cells are spread over a warp
+struct NodeShared {
+    uint32_t start[kNodeHalo * kNodeHalo * kNodeHaloZ], count[kNodeHalo * kNodeHalo * kNodeHaloZ];
+    uint16_t row[kNodeHalo * kNodeHaloZ];  // occupied cells of a row, a bit each
+    uint16_t list[kNodeThreads];           // nodes to search, a thread each
+    uint16_t hard[kNodeThreads];           // ... a warp each
+    double near2[kNodeCells];
+    int16_t cell[kNodeCells];              // offset in start and count
+    int n, nhard;
+};
+template <bool ORDER>
+__global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, const uint32_t* __restrict__ cell_start,
+                                                                const uint32_t* __restrict__ order,
+                                                                const __grid_constant__ NodeReach reach, double R2,
+                                                                double* __restrict__ out)
+{
+    __shared__ NodeShared sh;
+    const int nx = v.g.nx, ny = v.g.ny, nz = v.g.nz;
+    const int tile = (int)blockIdx.x >> 1;
+    const int tx = tile % v.g.tnx, ty = (tile / v.g.tnx) % v.g.tny, tz = tile / (v.g.tnx * v.g.tny);
+    const int x0 = tx * FE_TILE, y0 = ty * FE_TILE, z0 = tz * FE_TILE + ((int)blockIdx.x & 1) * kNodeLayers;
+    const double inv_bucket = 1.0 / v.bucket;
+
+    bool any = false;
+    if (threadIdx.x < 27) {
+        const int i = tx - 1 + (int)threadIdx.x % 3, j = ty - 1 + (int)threadIdx.x / 3 % 3, k = tz - 1 + (int)threadIdx.x / 9;
+        if ((unsigned)i < (unsigned)v.g.tnx && (unsigned)j < (unsigned)v.g.tny && (unsigned)k < (unsigned)v.g.tnz) {
+            const uint32_t first = (uint32_t)(i + v.g.tnx * (j + v.g.tny * k)) * FE_TILE_CELLS;
+            any = cell_start[first] != cell_start[first + FE_TILE_CELLS];
+        }
+    }
+    const bool occupied = __syncthreads_or(any);
+    if (occupied) {
+        for (int q = (int)threadIdx.x; q < kNodeHalo * kNodeHalo * kNodeHaloZ; q += kNodeThreads) {
+            const int i = x0 - 2 + q % kNodeHalo, j = y0 - 2 + q / kNodeHalo % kNodeHalo, k = z0 - 2 + q / (kNodeHalo * kNodeHalo);
+            uint32_t beg = 0, end = 0;
+            if ((unsigned)i < (unsigned)nx && (unsigned)j < (unsigned)ny && (unsigned)k < (unsigned)nz) {
+                const uint32_t key = (uint32_t)((i >> 3) + v.g.tnx * ((j >> 3) + v.g.tny * (k >> 3))) * FE_TILE_CELLS +
+                                     (uint32_t)((i & 7) + 8 * (j & 7) + 64 * (k & 7));
+                beg = cell_start[key];
+                end = cell_start[key + 1];
+            }
+            sh.start[q] = beg;
+            sh.count[q] = end - beg;
+        }
+        if (threadIdx.x < kNodeCells) {
+            const int c = (int)threadIdx.x;
+            const int w = c < 27 ? 0 : (c < 45 ? 1 : 2 + (c - 45) / 30);
+            int d[3];
+            node_cell(w, c - node_group_first(w), d);
+            sh.near2[c] = reach.near2[c];
+            sh.cell[c] = (int16_t)(d[0] + kNodeHalo * (d[1] + kNodeHalo * d[2]));
+        }
+        if (threadIdx.x == 0) sh.n = sh.nhard = 0;
+    }
+    __syncthreads();
+    if (occupied)
+        for (int r = (int)threadIdx.x; r < kNodeHalo * kNodeHaloZ; r += kNodeThreads) {
+            unsigned bits = 0;
+            for (int i = 0; i < kNodeHalo; ++i) bits |= sh.count[r * kNodeHalo + i] ? 1u << i : 0u;
+            sh.row[r] = (uint16_t)bits;
+        }
+    __syncthreads();
+    // occupied cells of group w around local node (lx, ly, lz) that reach into the band
+    auto group = [&](int w, int lx, int ly, int lz) {
+        const uint16_t* row = sh.row + ly + kNodeHalo * lz;  // of (dy, dz) = (-2, -2)
+        auto at = [&](int r) { return (unsigned)row[node_row(r) % 5 + kNodeHalo * (node_row(r) / 5)] >> lx; };
+        unsigned m = 0;
+        if (w < 2) {
+#pragma unroll
+            for (int r = 0; r < 9; ++r) {
+                const unsigned x = at(r);
+                m |= w == 0 ? ((x >> 1) & 7u) << (3 * r) : ((x & 1u) | ((x >> 3) & 2u)) << (2 * r);
+            }
+        } else if (w == 2) {
+#pragma unroll
+            for (int r = 0; r < 6; ++r) m |= (at(9 + r) & 31u) << (5 * r);
+        } else if (w == 3) {
+#pragma unroll
+            for (int r = 0; r < 6; ++r) m |= (at(15 + r) & 31u) << (5 * r);
+        } else {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) m |= (at(21 + r) & 31u) << (5 * r);
+        }
+        return m & reach.valid[w];
+    };
+
+    const double none = __longlong_as_double(0x7ff0000000000000ll);  // infinite: no particle within the band
+    auto value = [&](double best) { return __dsub_rn(best == none ? v.band : fmin(__dsqrt_rn(best), v.band), v.radius); };
+    auto bucket_ok = [&](double X, double Y, double Z, int i, int j, int k) {
+        return visited(v, bucket_fast(X, v.bucket, inv_bucket), bucket_fast(Y, v.bucket, inv_bucket),
+                       bucket_fast(Z, v.bucket, inv_bucket), i, j, k);
+    };
+    // the nearest of the particles in slots [s, s + n) by the reference's squared distance, if nearer than best
+    auto nearest = [&](uint32_t s, uint32_t n, double qx, double qy, double qz, double& best, uint32_t& arg) {
+        constexpr int B = 4;
+        for (uint32_t e = 0; e < n; e += B) {
+            uint32_t p[B];
+            float x[B], y[B], z[B];
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                const uint32_t at = s + min(e + b, n - 1);
+                p[b] = ORDER ? __ldg(order + at) : at;
+            }
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                x[b] = __ldg(v.px + p[b]);
+                y[b] = __ldg(v.py + p[b]);
+                z[b] = __ldg(v.pz + p[b]);
+            }
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                const double d2 = dist2_ref((double)x[b], (double)y[b], (double)z[b], qx, qy, qz);
+                if (d2 < best) {
+                    best = d2;
+                    arg = p[b];
+                }
+            }
+        }
+    };
+    const uint32_t nobody = 0xffffffffu;
+    // a node's value from the nearest particle found, or the node goes to the warps
+    auto finish = [&](int t, int i, int j, int k, double best, uint32_t arg) {
+        if (arg == nobody) best = none;
+        else if (!bucket_ok((double)__ldg(v.px + arg), (double)__ldg(v.py + arg), (double)__ldg(v.pz + arg), i, j, k)) {
+            sh.hard[atomicAdd(&sh.nhard, 1)] = (uint16_t)t;
+            return;
+        }
+        out[idx3(i, j, k, nx, ny)] = value(best);
+    };
+    const double beyond = __longlong_as_double(__double_as_longlong(R2) + 1);  // the next double: best <= R2 counts
+
+    {
+        const int t = (int)threadIdx.x;
+        const int lx = t & 7, ly = (t >> 3) & 7, lz = t >> 6;
+        const int i = x0 + lx, j = y0 + ly, k = z0 + lz;
+        if (i < nx && j < ny && k < nz) {
+            double best = beyond;
+            uint32_t arg = nobody;
+            bool more = false;
+            if (occupied) {
+                const int q = lx + 2 + kNodeHalo * (ly + 2 + kNodeHalo * (lz + 2));
+                const uint32_t n = sh.count[q];
+                if (n > 0 && n <= kNodeLaneCap) nearest(sh.start[q], n, v.q_pos[0][i], v.q_pos[1][j], v.q_pos[2][k], best, arg);
+                if (!(best <= reach.own2)) {
+                    unsigned m = 0;
+#pragma unroll
+                    for (int w = 0; w < kNodeGroups; ++w) m |= group(w, lx, ly, lz);
+                    more = m != 0;
+                }
+            }
+            if (more) sh.list[atomicAdd(&sh.n, 1)] = (uint16_t)t;
+            else finish(t, i, j, k, best, arg);
+        }
+    }
+    if (!occupied) return;
+    __syncthreads();
+
+    if ((int)threadIdx.x < sh.n) {
+        const int t = sh.list[threadIdx.x];
+        const int lx = t & 7, ly = (t >> 3) & 7, lz = t >> 6;
+        const int i = x0 + lx, j = y0 + ly, k = z0 + lz;
+        const int q0 = lx + 2 + kNodeHalo * (ly + 2 + kNodeHalo * (lz + 2));
+        const double qx = v.q_pos[0][i], qy = v.q_pos[1][j], qz = v.q_pos[2][k];
+        double best = beyond;
+        uint32_t arg = nobody;
+        bool full = false;
+        for (int w = 0; w < kNodeGroups; ++w) {
+            if (!(reach.group2[w] < best)) continue;
+            const int first = node_group_first(w);
+            for (unsigned m = group(w, lx, ly, lz); m; m &= m - 1) {
+                const int c = first + __ffs(m) - 1;
+                if (!(sh.near2[c] < best)) continue;
+                const int q = q0 + sh.cell[c];
+                const uint32_t n = sh.count[q];
+                if (n <= kNodeLaneCap) nearest(sh.start[q], n, qx, qy, qz, best, arg);
+                else full = true;
+            }
+        }
+        if (full) sh.hard[atomicAdd(&sh.nhard, 1)] = (uint16_t)t;
+        else finish(t, i, j, k, best, arg);
+    }
+    __syncthreads();
+
+    // the particle of slot s against node (i, j, k) at (qx, qy, qz): the reference's squared distance and bucket tests
+    auto test = [&](uint32_t s, int i, int j, int k, double qx, double qy, double qz, double& best) {
+        const uint32_t p = ORDER ? __ldg(order + s) : s;
+        const double X = (double)__ldg(v.px + p), Y = (double)__ldg(v.py + p), Z = (double)__ldg(v.pz + p);
+        const double d2 = dist2_ref(X, Y, Z, qx, qy, qz);
+        if (d2 < best && d2 <= R2 && bucket_ok(X, Y, Z, i, j, k)) best = d2;
+    };
+    const int lane = (int)threadIdx.x & 31;
+    for (int e = (int)threadIdx.x >> 5; e < sh.nhard; e += kNodeThreads >> 5) {
+        const int t = sh.hard[e];
+        const int lx = t & 7, ly = (t >> 3) & 7, lz = t >> 6;
+        const int i = x0 + lx, j = y0 + ly, k = z0 + lz;
+        const double qx = v.q_pos[0][i], qy = v.q_pos[1][j], qz = v.q_pos[2][k];
+        double best = none;
+        for (int first = 0; first < kNodeCells; first += 32) {  // each lane its cell
+            const int c = first + lane;
+            uint32_t s = 0, n = 0;
+            if (c < kNodeCells && sh.near2[c] < best) {
+                const int q = lx + 2 + kNodeHalo * (ly + 2 + kNodeHalo * (lz + 2)) + sh.cell[c];
+                s = sh.start[q];
+                n = sh.count[q];
+            }
+            if (n <= kNodeLaneCap)
+                for (uint32_t m = 0; m < n; ++m) test(s + m, i, j, k, qx, qy, qz, best);
+            unsigned full = __ballot_sync(0xffffffffu, n > kNodeLaneCap);
+            while (full) {
+                const int from = __ffs(full) - 1;
+                full &= full - 1;
+                const uint32_t fs = __shfl_sync(0xffffffffu, s, from), fn = __shfl_sync(0xffffffffu, n, from);
+                for (uint32_t m = (uint32_t)lane; m < fn; m += 32) test(fs + m, i, j, k, qx, qy, qz, best);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) best = fmin(best, __shfl_xor_sync(0xffffffffu, best, o));
+        }
+        if (lane == 0) out[idx3(i, j, k, nx, ny)] = value(best);
+    }
 }
 
 // BackwardEulerDiffusionSolver::BuildX/Y/ZMarkers (fluid_solvers/backward_euler_diffusion_solver.cpp:71-128):
@@ -464,9 +732,8 @@ __global__ void k_face_mark(SceneView v, DiffWork d)
     const double fx = d.tab_f[base + fc.i], fy = d.tab_f[base + d.tab_stride + fc.j];
     const double fz = d.tab_f[base + 2 * d.tab_stride + fc.k];
     const int ip = min(i0 + 1, nx - 1), jp = min(j0 + 1, ny - 1), kp = min(k0 + 1, nz - 1);
-    const unsigned long long* __restrict__ node = d.node_dist;
-    // node value min(2r, sqrt(smallest squared distance)) - r (all ones: no particle within the band)
-    auto val = [&](int i, int j, int k) { return node_value(__ldg(node + idx3(i, j, k, nx, ny)), v.band, v.radius); };
+    const double* __restrict__ node = d.node;
+    auto val = [&](int i, int j, int k) { return __ldg(node + idx3(i, j, k, nx, ny)); };
     const double c000 = val(i0, j0, k0), c100 = val(ip, j0, k0), c010 = val(i0, jp, k0), c110 = val(ip, jp, k0);
     const double c001 = val(i0, j0, kp), c101 = val(ip, j0, kp), c011 = val(i0, jp, kp), c111 = val(ip, jp, kp);
     const double b0 = lerp_ref(lerp_ref(c000, c100, fx), lerp_ref(c010, c110, fx), fy);
@@ -562,29 +829,73 @@ cudaError_t launch_fluid_sdf(const SceneView& v, double* out, cudaStream_t st)
     return cudaGetLastError();
 }
 
-cudaError_t launch_node_sdf(const SceneView& v, unsigned long long* node, double* sdf, cudaStream_t st)
+// Cells up to two away hold every particle of a node's band, by the squared distances from a node (the centre of its cell) to
+// the nearest points of other cells.  A particle may be listed in the cell next to its own when it is within the FP32
+// rounding of their border, and in an outer cell when it is outside the grid (then it is further away than the cell).
+// False when the band is wider than that.
+static bool node_reach(const SceneView& v, NodeReach& r)
+{
+    const double R2 = v.band * v.band;
+    bool ok = true;
+    double near2[3][3];
+    r.own2 = HUGE_VAL;
+    for (int a = 0; a < 3; ++a) {
+        const double delta = 1e-6 * (std::fabs(v.origin[a]) + 4.0 * v.size[a]);
+        for (int d = 0; d < 3; ++d) {
+            const double near = std::max(0.0, (d - 0.5) * v.h[a] - delta);
+            near2[a][d] = near * near;
+        }
+        r.own2 = std::min(r.own2, near2[a][1]);
+        ok = ok && v.band < 2.5 * v.h[a] - delta && delta < 0.1 * v.h[a];
+    }
+    for (int w = 0; w < kNodeGroups; ++w) {
+        r.group2[w] = HUGE_VAL;
+        r.valid[w] = 0;
+        const int first = node_group_first(w), end = w + 1 < kNodeGroups ? node_group_first(w + 1) : kNodeCells;
+        for (int c = first; c < end; ++c) {
+            int d[3];
+            node_cell(w, c - first, d);
+            r.near2[c] = near2[0][std::abs(d[0])] + near2[1][std::abs(d[1])] + near2[2][std::abs(d[2])];
+            r.group2[w] = std::min(r.group2[w], r.near2[c]);
+            if (r.near2[c] <= R2) r.valid[w] |= 1u << (c - first);
+        }
+    }
+    return ok;
+}
+
+bool node_sdf_uses_cells(const SceneView& v)
+{
+    NodeReach r;
+    return v.np > 0 && node_reach(v, r);
+}
+
+cudaError_t launch_node_sdf(const SceneView& v, const NodeCells& cells, double* sdf, cudaStream_t st)
 {
     const size_t nc = (size_t)v.g.nx * v.g.ny * v.g.nz;
-    cudaError_t e = cudaMemsetAsync(node, 0xff, nc * sizeof(unsigned long long), st);
+    const double R2 = v.band * v.band;
+    NodeReach r;
+    if (v.np > 0 && cells.start && node_reach(v, r)) {
+        const unsigned blocks = 2u * (unsigned)(v.g.tnx * v.g.tny * v.g.tnz);
+        if (cells.order) k_sdf_gather<true><<<blocks, kNodeThreads, 0, st>>>(v, cells.start, cells.order, r, R2, sdf);
+        else k_sdf_gather<false><<<blocks, kNodeThreads, 0, st>>>(v, cells.start, nullptr, r, R2, sdf);
+        count_launch();
+        return cudaGetLastError();
+    }
+    cudaError_t e = cudaMemsetAsync(sdf, 0xff, nc * sizeof(double), st);
     if (e != cudaSuccess) return e;
     if (v.np > 0) {
-        k_sdf_scatter<<<(unsigned)((v.np + 255) / 256), 256, 0, st>>>(v, node, v.band * v.band);
+        k_sdf_scatter<<<(unsigned)((v.np + 255) / 256), 256, 0, st>>>(v, reinterpret_cast<unsigned long long*>(sdf), R2);
         count_launch();
     }
-    k_node_values<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(node, nc, v.band, v.radius, sdf);
+    k_node_values<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(sdf, nc, v.band, v.radius);
     count_launch();
     return cudaGetLastError();
 }
 
-cudaError_t launch_face_fluid_marks(const SceneView& v, const DiffWork& d, cudaStream_t st)
+cudaError_t launch_face_fluid_marks(const SceneView& v, const NodeCells& cells, const DiffWork& d, cudaStream_t st)
 {
-    const size_t nc = (size_t)v.g.nx * v.g.ny * v.g.nz;
-    cudaError_t e = cudaMemsetAsync(d.node_dist, 0xff, nc * sizeof(unsigned long long), st);
+    cudaError_t e = launch_node_sdf(v, cells, d.node, st);
     if (e != cudaSuccess) return e;
-    if (v.np > 0) {
-        k_sdf_scatter<<<(unsigned)((v.np + 255) / 256), 256, 0, st>>>(v, d.node_dist, v.band * v.band);
-        count_launch();
-    }
     k_face_mark<<<face_grid(v.g.nx, v.g.ny, v.g.nz), dim3(kTileX, kTileY), 0, st>>>(v, d);
     count_launch();
     return cudaGetLastError();

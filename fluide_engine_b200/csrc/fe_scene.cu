@@ -142,6 +142,7 @@ struct fe_scene {
         double* sdf = nullptr;
         uint8_t* cfg = nullptr;
         uint32_t *nvert = nullptr, *ntri = nullptr, *vbase = nullptr, *tbase = nullptr;
+        uint32_t *cell_count = nullptr, *cell_start = nullptr;  // the particles by cell, for the SDF
         void* tmp = nullptr;
         size_t tmp_bytes = 0, items = 0;
         double *V = nullptr, *N = nullptr;
@@ -349,7 +350,7 @@ fe_status alloc_diffusion(fe_scene* s)
     const int dev = s->device;
     cudaStream_t st = s->own_stream;
     DiffWork d{};
-    FE_CUDA(dalloc(L, &d.node_dist, nc, dev, st));
+    FE_CUDA(dalloc(L, &d.node, nc, dev, st));
     FE_CUDA(dalloc(L, &d.mark, nf, dev, st));
     FE_CUDA(cudaMemsetAsync(d.mark, 0, nf, st));
     FE_CUDA(dalloc(L, &d.list, nf, dev, st));
@@ -713,6 +714,9 @@ double inner_tol(const fe_scene_desc& d, bool multigrid)
     return std::min(1e-2, std::max(1e-4, std::pow(d.cg_rel_tol, 1.0 / k)));
 }
 
+// The current particles' cells, while they are known.
+NodeCells node_cells(const fe_scene* s) { return {s->cells_current ? s->base.cell_start : nullptr, nullptr}; }
+
 fe_status enqueue_steps(fe_scene* s, double dt, int first, int last, cudaStream_t stream = nullptr)
 {
     cudaStream_t st = stream ? stream : s->stream;
@@ -735,7 +739,7 @@ fe_status enqueue_steps(fe_scene* s, double dt, int first, int last, cudaStream_
             s->grid_cur = 0;
             break;
         case kStepMark:
-            if (s->colliders.count > 0) FE_CUDA(launch_collider_marks(v, s->cw, s->surf.node, &s->collider_fluid_sdf, st));
+            if (s->colliders.count > 0) FE_CUDA(launch_collider_marks(v, node_cells(s), s->cw, &s->collider_fluid_sdf, st));
             else FE_CUDA(launch_mark(v, s->cells_current, st));
             break;
         case kStepPre:
@@ -765,8 +769,8 @@ fe_status enqueue_steps(fe_scene* s, double dt, int first, int last, cudaStream_
             if (s->desc.viscosity > 0.0) {
                 const int pb = pressure_buffer(s);
                 FE_CUDA(ensure_grid(s, pb, st));
-                FE_CUDA(launch_diffuse(v, s->diff, s->cg, pb ? v.u2 : v.u, pb ? v.v2 : v.v, pb ? v.w2 : v.w, dt,
-                                       s->desc.viscosity, st));
+                FE_CUDA(launch_diffuse(v, node_cells(s), s->diff, s->cg, pb ? v.u2 : v.u, pb ? v.v2 : v.v, pb ? v.w2 : v.w,
+                                       dt, s->desc.viscosity, st));
             }
             break;
         case kStepRhs:
@@ -1031,7 +1035,7 @@ fe_status surf_alloc(fe_scene* s)
         FE_CUDA(cudaStreamSynchronize(s->stream));
         w.items = mc_items(b.g.nx, b.g.ny, b.g.nz);
         if (w.items + 1 >= (1ull << 32)) return set_error(FE_ERR_BAD_ARG, "grid too large for surface extraction");
-        w.tmp_bytes = sort_scan_tmp_bytes((uint32_t)w.items);
+        w.tmp_bytes = std::max(sort_scan_tmp_bytes((uint32_t)w.items), sort_scan_tmp_bytes(b.g.key_space));
         auto& L = s->allocs;
         FE_CUDA(dalloc(L, &w.node, nc, s->device, st));
         FE_CUDA(dalloc(L, &w.sdf, nc, s->device, st));
@@ -1040,6 +1044,8 @@ fe_status surf_alloc(fe_scene* s)
         FE_CUDA(dalloc(L, &w.ntri, w.items, s->device, st));
         FE_CUDA(dalloc(L, &w.vbase, w.items + 1, s->device, st));
         FE_CUDA(dalloc(L, &w.tbase, w.items + 1, s->device, st));
+        FE_CUDA(dalloc(L, &w.cell_count, b.g.key_space, s->device, st));
+        FE_CUDA(dalloc(L, &w.cell_start, (size_t)b.g.key_space + 1, s->device, st));
         uint8_t* tmp;
         FE_CUDA(dalloc(L, &tmp, w.tmp_bytes, s->device, st));
         w.tmp = tmp;
@@ -1062,8 +1068,21 @@ fe_status surface_sdf(fe_scene* s)
                                 s->stream));
         return FE_OK;
     }
-    const SceneView v = view_of(s, s->prev_valid ? (s->parity ^ 1) : s->parity);
-    FE_CUDA(launch_node_sdf(v, s->surf.node, s->surf.sdf, s->stream));
+    SceneView v = view_of(s, s->prev_valid ? (s->parity ^ 1) : s->parity);
+    NodeCells cells{nullptr, nullptr};
+    if (node_sdf_uses_cells(v)) {
+        // these particles are in the order of an earlier sort or of the caller: grouped by cell in the staging buffer (9
+        // words a particle) and cell arrays of the surface's own, so the last sort's stay as they are
+        auto& w = s->surf;
+        v.key = reinterpret_cast<uint32_t*>(s->staging);
+        v.rank = v.key + v.np;
+        v.perm = v.rank + v.np;
+        v.cell_count = w.cell_count;
+        v.cell_start = w.cell_start;
+        FE_CUDA(launch_group(v, s->stream, w.tmp, w.tmp_bytes));
+        cells = {v.cell_start, v.perm};
+    }
+    FE_CUDA(launch_node_sdf(v, cells, s->surf.sdf, s->stream));
     return FE_OK;
 }
 
@@ -2021,7 +2040,7 @@ fe_status fe_scene_add_mesh_collider(fe_scene* s, const double* vertices, uint64
         if (tri[4 * t + 3] < 0 || (uint64_t)tri[4 * t + 3] >= n_normals)
             return set_error(FE_ERR_BAD_ARG, "triangle %llu has normal id %lld of %llu", (unsigned long long)t,
                              (long long)tri[4 * t + 3], (unsigned long long)n_normals);
-    fe_status r = surf_alloc(s);  // its node scratch serves the band SDF of the collider marks
+    fe_status r = surf_alloc(s);  // its node scratch serves the collider's own SDF
     if (r != FE_OK) return r;
     std::vector<void*> allocs;
     double* dV = nullptr;

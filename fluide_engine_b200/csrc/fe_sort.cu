@@ -426,7 +426,7 @@ cudaError_t launch_exclusive_scan(const uint32_t* in, uint32_t n, uint32_t* out,
     return cudaGetLastError();
 }
 
-cudaError_t launch_sort(const SceneView& v, cudaStream_t st, void* scan_tmp, size_t scan_tmp_bytes)
+cudaError_t launch_group(const SceneView& v, cudaStream_t st, void* scan_tmp, size_t scan_tmp_bytes)
 {
     const uint32_t K = v.g.key_space;
     cudaError_t e = cudaMemsetAsync(v.cell_count, 0, (size_t)K * sizeof(uint32_t), st);
@@ -445,12 +445,22 @@ cudaError_t launch_sort(const SceneView& v, cudaStream_t st, void* scan_tmp, siz
     k_scan_final<<<nb, kScanThreads, 0, st>>>(v.cell_count, K, sums, v.cell_start);
     count_launch(3);
     if (v.np > 0) {
-        uint32_t* long_count = sums + nb + 1;
-        k_place<<<pb, T, 0, st>>>(v, long_count);
-        k_cellrank<<<pb, T, 0, st>>>(v, long_count);
-        k_bigcell<<<kBigCellBlocks, 1024, 0, st>>>(v, long_count);
-        count_launch(3);
+        k_place<<<pb, T, 0, st>>>(v, sums + nb + 1);
+        count_launch();
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sort(const SceneView& v, cudaStream_t st, void* scan_tmp, size_t scan_tmp_bytes)
+{
+    cudaError_t e = launch_group(v, st, scan_tmp, scan_tmp_bytes);
+    if (e != cudaSuccess || v.np == 0) return e;
+    const int T = 256;
+    const unsigned pb = (unsigned)((v.np + (uint64_t)T * kSortBatch - 1) / ((uint64_t)T * kSortBatch));
+    uint32_t* long_count = (uint32_t*)scan_tmp + (v.g.key_space + kScanTile - 1) / kScanTile + 1;
+    k_cellrank<<<pb, T, 0, st>>>(v, long_count);
+    k_bigcell<<<kBigCellBlocks, 1024, 0, st>>>(v, long_count);
+    count_launch(2);
     return cudaGetLastError();
 }
 
