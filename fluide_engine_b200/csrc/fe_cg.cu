@@ -197,6 +197,7 @@ __device__ __forceinline__ void cg_body(SolverSmem& smem, const SceneView& v, co
 __global__ void __launch_bounds__(kCgThreads, 1) k_cg(SceneView v, CgWork w, CgParams prm)
 {
     __shared__ SolverSmem smem;
+    if (gated_off(prm)) return;
     cluster_begin(w, smem.sh);
     cg_body(smem, v, w, prm, blockIdx.x, gridDim.x);
     solver_exit(w, gridDim.x);
@@ -211,6 +212,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) k_mgcg(SceneView v, CgWork w, M
 {
     __shared__ MgShared ms;
     extern __shared__ __align__(16) unsigned char mg_dynamic[];
+    if (gated_off(prm)) return;
     cluster_begin(w, ms.sh);
     const int tiles = tiles_of(v.g.nx) * tiles_of(v.g.ny) * tiles_of(v.g.nz);
     const int nblk = w.cluster > 1 ? (int)gridDim.x : min((int)gridDim.x, tiles);
@@ -455,9 +457,10 @@ int mg_block_from(const MgLevel* lv, int levels, int block_cells)
 }
 
 cudaError_t launch_mgcg(const SceneView& v, const CgWork& w, const MgWork& mg, double rel_tol, double inner_tol,
-                        int max_it, int max_refine, cudaStream_t st)
+                        int max_it, int max_refine, cudaStream_t st, const uint32_t* gate)
 {
     CgParams prm;
+    prm.gate = gate;
     prm.rel_tol = rel_tol;
     prm.inner_tol = inner_tol;
     prm.max_it = max_it;
@@ -485,9 +488,11 @@ cudaError_t launch_mgcg(const SceneView& v, const CgWork& w, const MgWork& mg, d
 }
 
 cudaError_t launch_cg(const SceneView& v, const CgWork& w, double rel_tol, double inner_tol, int max_it,
-                      int max_refine, cudaStream_t st)
+                      int max_refine, cudaStream_t st, const uint32_t* gate)
 {
     CgParams prm;
+    prm.gate = gate;
+    prm.gate_on = true;
     prm.rel_tol = rel_tol;
     prm.inner_tol = inner_tol;
     prm.max_it = max_it;

@@ -601,26 +601,41 @@ __device__ __forceinline__ uint32_t find_root(const uint32_t* label, uint32_t x,
     return x;
 }
 
-__global__ void k_ccl_init(const uint8_t* __restrict__ marks, size_t nc, uint32_t* __restrict__ label,
-                           uint8_t* __restrict__ open_comp, double* __restrict__ sum, uint32_t* __restrict__ cnt)
+// A cell's first label is the first cell of its run of FLUID cells along x within the warp's 32 cells.
+__global__ void k_ccl_init(const uint8_t* __restrict__ marks, size_t nc, int nx, uint32_t* __restrict__ label,
+                           uint8_t* __restrict__ open_comp, double* __restrict__ sum, uint32_t* __restrict__ cnt,
+                           uint32_t* __restrict__ enclosed)
 {
-    for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < nc; c += (size_t)gridDim.x * blockDim.x) {
-        label[c] = marks[c] == FE_CELL_FLUID ? (uint32_t)c : kNoLabel;
+    const int lane = (int)threadIdx.x & 31;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t c0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x - lane; c0 < nc; c0 += stride) {
+        const size_t c = c0 + lane;
+        const bool fluid = c < nc && marks[c] == FE_CELL_FLUID;
+        const unsigned fluids = __ballot_sync(0xffffffffu, fluid);
+        const unsigned starts = __ballot_sync(0xffffffffu, fluid && c % nx == 0) | (fluids & ~(fluids << 1));
+        if (c >= nc) continue;
+        const unsigned upto = starts & (0xffffffffu >> (31 - lane));
+        label[c] = fluid ? (uint32_t)(c0 + (31 - __clz((int)upto))) : kNoLabel;
         open_comp[c] = 0;
         sum[c] = 0.0;
         cnt[c] = 0u;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *enclosed = 0u;
 }
 
+// Links along y and z, once per stretch of neighbouring pairs along x (the pairs before it are linked through their own
+// runs), and along x where a run goes on in the next warp's cells.  56 us with a link per pair of cells at 64^3.
 __global__ void k_ccl_union(const uint8_t* __restrict__ marks, int nx, int ny, int nz, uint32_t* label, int* err)
 {
     const size_t nc = (size_t)nx * ny * nz, sxy = (size_t)nx * ny;
     for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < nc; c += (size_t)gridDim.x * blockDim.x) {
         if (marks[c] != FE_CELL_FLUID) continue;
         const int i = (int)(c % nx), j = (int)((c / nx) % ny), k = (int)(c / sxy);
-        const size_t nb[3] = {i > 0 ? c - 1 : c, j > 0 ? c - nx : c, k > 0 ? c - sxy : c};
+        const bool left = i > 0 && marks[c - 1] == FE_CELL_FLUID;
+        const size_t nb[3] = {left && (threadIdx.x & 31) == 0 ? c - 1 : c, j > 0 ? c - nx : c, k > 0 ? c - sxy : c};
         for (int q = 0; q < 3; ++q) {
             if (nb[q] == c || marks[nb[q]] != FE_CELL_FLUID) continue;
+            if (q > 0 && left && marks[nb[q] - 1] == FE_CELL_FLUID) continue;
             uint32_t a = (uint32_t)c, b = (uint32_t)nb[q];
             for (int it = 0; it < kFindLimit; ++it) {
                 a = find_root(label, a, err);
@@ -671,13 +686,14 @@ __global__ void k_ccl_sums(const uint8_t* __restrict__ marks, const double* __re
 // consistent system unchanged and makes an inconsistent one solvable.
 __global__ void k_ccl_project(const uint8_t* __restrict__ marks, size_t nc, const uint32_t* __restrict__ label,
                               const uint8_t* __restrict__ open_comp, const double* __restrict__ sum,
-                              const uint32_t* __restrict__ cnt, double* __restrict__ b)
+                              const uint32_t* __restrict__ cnt, double* __restrict__ b, uint32_t* enclosed)
 {
     for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < nc; c += (size_t)gridDim.x * blockDim.x) {
         if (marks[c] != FE_CELL_FLUID) continue;
         const uint32_t r = label[c];
         if (open_comp[r]) continue;
         b[c] -= sum[r] / (double)cnt[r];
+        if (cnt[r] > 1u) *enclosed = 1u;
     }
 }
 
@@ -714,7 +730,7 @@ cudaError_t launch_collider_project_rhs(const SceneView& v, const CollideWork& w
 {
     const int nx = v.g.nx, ny = v.g.ny, nz = v.g.nz;
     const size_t nc = (size_t)nx * ny * nz;
-    k_ccl_init<<<node_blocks(nc), 256, 0, st>>>(v.marks, nc, w.label, w.open_comp, w.comp_sum, w.comp_cnt);
+    k_ccl_init<<<node_blocks(nc), 256, 0, st>>>(v.marks, nc, nx, w.label, w.open_comp, w.comp_sum, w.comp_cnt, w.enclosed);
     count_launch();
     k_ccl_union<<<node_blocks(nc), 256, 0, st>>>(v.marks, nx, ny, nz, w.label, err);
     count_launch();
@@ -722,7 +738,8 @@ cudaError_t launch_collider_project_rhs(const SceneView& v, const CollideWork& w
     count_launch();
     k_ccl_sums<<<node_blocks(nc), 256, 0, st>>>(v.marks, v.b, nc, w.label, w.open_comp, w.comp_sum, w.comp_cnt);
     count_launch();
-    k_ccl_project<<<node_blocks(nc), 256, 0, st>>>(v.marks, nc, w.label, w.open_comp, w.comp_sum, w.comp_cnt, v.b);
+    k_ccl_project<<<node_blocks(nc), 256, 0, st>>>(v.marks, nc, w.label, w.open_comp, w.comp_sum, w.comp_cnt, v.b,
+                                                 w.enclosed);
     count_launch();
     return cudaGetLastError();
 }

@@ -361,10 +361,11 @@ struct MultiCgScene {
 cudaError_t multi_cg_capacity(int device, int* max_blocks, int* threads);
 // Re-splits total_blocks among the S scenes in proportion to their last solve's work, then solves them.
 cudaError_t launch_multi_cg(MultiCgScene* scenes, int S, int total_blocks, cudaStream_t st);
+// gate: a word on the device; launch_mgcg solves when it is zero, launch_cg when it is not (null: always).
 cudaError_t launch_cg(const SceneView& v, const CgWork& w, double rel_tol, double inner_tol, int max_it, int max_refine,
-                      cudaStream_t st);
+                      cudaStream_t st, const uint32_t* gate = nullptr);
 cudaError_t launch_mgcg(const SceneView& v, const CgWork& w, const MgWork& mg, double rel_tol, double inner_tol,
-                        int max_it, int max_refine, cudaStream_t st);
+                        int max_it, int max_refine, cudaStream_t st, const uint32_t* gate = nullptr);
 
 // Surface extraction (fe_surface.cu): items = the node grid's cubes, then its XY, YZ and XZ cap squares (two faces
 // each); counts per item, then the mesh from the scanned counts.
@@ -431,6 +432,7 @@ struct CollideWork {
     uint8_t* open_comp;      // n^3 (by root): the component has an AIR neighbour
     double* comp_sum;        // n^3 (by root): right-hand-side sum of the component
     uint32_t* comp_cnt;      // n^3 (by root): its cells
+    uint32_t* enclosed;      // 1: a component of two or more cells has no AIR neighbour
     // collision response (sized by the particle capacity)
     float* start;            // 3 per slot: position before the move
     float* startv;           // 3 per slot: velocity before the move (after the grid-to-particle transfer)

@@ -8,7 +8,8 @@
 // on the same FP64 residual test).
 //
 // Hierarchy: level l >= 1 halves every axis of level l-1 (rounding up) until the largest axis is <= 8.  phi, the
-// fluid fraction of a coarse cell, is the mean of its children's; a coarse cell is in the system when phi > kMaskPhi.
+// fluid fraction of a coarse cell, is the mean of its children's, BOUNDRY cells left out; a coarse cell is in the system when
+// phi > kMaskPhi, and one of nothing but BOUNDRY cells is a wall.
 // Its operator is the 7-point matrix with spacing 2^l h, except that the coefficient toward a cell outside the system
 // is h_l^-2 / d, d the distance (in h_l) from the cell's centre to the air value (0) as the fractions put it:
 // half the fluid of the cell's own half on that side, all of the neighbour's, and half a level-0 cell.  A coarse cell
@@ -793,6 +794,7 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
         LB = max(LB, max(fit, 1));
     }
     unsigned gen = 0;
+    const bool solids = prm.gate != nullptr;  // a scene with colliders: there may be BOUNDRY cells
 
     if (threadIdx.x < 128) {
         const int m = (int)threadIdx.x;
@@ -828,12 +830,12 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
         for (int it = 0; it < 512 / MANY; ++it) {
             const int q = lt + it * MANY;
             const int i = tx * 8 + (q & 7), j = ty * 8 + ((q >> 3) & 7), k = tz * 8 + (q >> 6);
-            float phi = -1.f;  // outside the grid
+            float phi = -1.f;  // outside the grid, or no part of the system as a wall is none
             if (i < nx && j < ny && k < nz) {
                 const size_t c = (size_t)i + (size_t)nx * j + sxy * k;
                 const uint32_t m = solve_mask(v.marks, (int)c, i, j, k, nx, ny, nz);
                 code[c] = (uint8_t)m;
-                phi = m ? 1.f : 0.f;
+                phi = m ? 1.f : (solids && v.marks[c] != FE_CELL_AIR ? -1.f : 0.f);
                 if (m) {
                     acc2[0] += b[c] * b[c];
                     acc2[1] += 1.0;
@@ -904,7 +906,7 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
                         child[d] = -1.f;
                         if (i < Fl.nx && j < Fl.ny && k < Fl.nz) {
                             const size_t f = (size_t)i + (size_t)Fl.nx * ((size_t)j + (size_t)Fl.ny * (size_t)k);
-                            child[d] = l == 1 ? (__ldcg(code + f) ? 1.f : 0.f) : __ldcg(Fl.t + f);
+                            child[d] = l > 1 ? __ldcg(Fl.t + f) : (__ldcg(code + f) ? 1.f : (solids && v.marks[f] != FE_CELL_AIR ? -1.f : 0.f));
                         }
                     }
                     float diag = 0.f;
@@ -915,6 +917,7 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
                             const int n = g[a] + (side ? 1 : -1);
                             if (n < 0 || n >= cn[a]) continue;  // wall: no flux
                             const float phi = __ldcg(C.t + (side ? c + st[a] : c - st[a]));
+                            if (phi < 0.f) continue;  // nothing but BOUNDRY: a wall
                             float coef = 1.f;
                             if (!(phi > kMaskPhi)) {
                                 float sum = 0.f, cnt = 0.f;
@@ -950,10 +953,13 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
             for (int d = 0; d < 8; ++d) {
                 const int i = 2 * I + (d & 1), j = 2 * J + ((d >> 1) & 1), k = 2 * K + (d >> 2);
                 if (i >= Fl.nx || j >= Fl.ny || k >= Fl.nz) continue;
-                sum += __ldcg(Fl.t + ((size_t)i + (size_t)Fl.nx * ((size_t)j + (size_t)Fl.ny * (size_t)k)));
-                cnt += 1.f;
+                const float x = __ldcg(Fl.t + ((size_t)i + (size_t)Fl.nx * ((size_t)j + (size_t)Fl.ny * (size_t)k)));
+                if (x >= 0.f) {
+                    sum += x;
+                    cnt += 1.f;
+                }
             }
-            C.t[t] = sum / cnt;
+            C.t[t] = cnt > 0.f ? sum / cnt : -1.f;
         }
         __threadfence();
         __syncthreads();

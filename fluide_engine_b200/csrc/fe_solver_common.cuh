@@ -26,7 +26,10 @@ struct CgParams {
     fe_step_stats* stats_ring;
     unsigned* stats_counter;
     unsigned stats_cap;
+    const uint32_t* gate = nullptr;  // the kernel runs only when this word is zero (gate_on: only when it is not)
+    bool gate_on = false;
 };
+__device__ __forceinline__ bool gated_off(const CgParams& prm) { return prm.gate && (*prm.gate != 0u) != prm.gate_on; }
 
 // ---- Grid barrier.  The barrier words and the totals start every launch at zero: the last block to leave a
 // solver kernel puts them back (solver_exit), and the host clears them after a solve that failed.  bar[0] counts

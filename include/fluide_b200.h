@@ -337,7 +337,7 @@ fe_status fe_scene_get_tuning(fe_scene* s, fe_tuning* t);
  * a given family does not depend on that. */
 enum { FE_TUNE_ALL = 0, FE_TUNE_SHAPE = 1 };
 /* The autotuner: times every candidate launch choice of the scene's pressure solve -- the plain CG at 256 / 512 /
- * 1024 threads per block, alone or in clusters of 2 blocks, and (grids with a multigrid hierarchy, no colliders)
+ * 1024 threads per block, alone or in clusters of 2 blocks, and (grids with a multigrid hierarchy)
  * the multigrid-preconditioned CG at 512 / 1024 threads with one-block levels up to 2048 or 4096 cells; with
  * FE_TUNE_SHAPE only the current family's --
  * over `substeps` substeps of dt each from the scene's current state (CUDA events on the scene's stream,
