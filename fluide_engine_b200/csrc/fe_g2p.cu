@@ -15,65 +15,112 @@
 namespace fe {
 namespace {
 
+// Stencil of a point on one staggered grid: the first face of each axis' pair and the fractions.  A pair is always two
+// neighbouring faces: GetBarycentric's clamps keep the first one below the last face, and no axis has fewer than two.
+struct Corner {
+    int i, j, k;
+    float fx, fy, fz;
+};
+
+// Two FP32 values in a register pair: the packed multiply and FMA take one instruction for both.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 pack2(float a, float b)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(F2 s, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(s)); }
+// (1 - f) a + f b of both, m = (1 - f, 1 - f) and f2 = (f, f)
+__device__ __forceinline__ F2 lerp2(F2 a, F2 b, F2 m, F2 f2)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(m), "l"(a));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f2), "l"(b), "l"(r));
+    return r;
+}
+
 // Face values of the six arrays a transfer reads (u, v, w and the FLIP snapshot su, sv, sw).
 struct FaceSource {
     const float* g[6];          // u, v, w, su, sv, sw
     int sx[3], sy[3];           // face-array sizes of the components (x, y)
-    // Offset of corner (i, j, k) of component comp's stencil and the steps to its other corners (0 where the stencil
-    // is clamped onto one face): one 64-bit index, then 32-bit steps (a step spans at most one plane of faces).
-    __device__ __forceinline__ size_t corner_base(int comp, const Stencil& st, int& dx, int& dy, int& dz) const
+    __device__ __forceinline__ size_t corner_base(int comp, const Corner& st) const
     {
-        dx = st.ip - st.i;
-        dy = (st.jp - st.j) * sx[comp];
-        dz = (st.kp - st.k) * sx[comp] * sy[comp];
         return idx3(st.i, st.j, st.k, sx[comp], sy[comp]);
     }
-    // the 8 corner values of array a from its base, in the reference's corner order (x fastest)
-    __device__ __forceinline__ void load8(int a, size_t base, int dx, int dy, int dz, float c[8]) const
+    // the 8 corner values of array a from its base, in the reference's corner order (x fastest): four rows of two
+    __device__ __forceinline__ void load8(int a, size_t base, float c[8]) const
     {
         const float* p = g[a] + base;
+        const float* q = p + sx[a % 3];
+        const float* r = p + (size_t)sx[a % 3] * (size_t)sy[a % 3];
+        const float* t = q + (size_t)sx[a % 3] * (size_t)sy[a % 3];
         c[0] = __ldg(p);
-        c[1] = __ldg(p + dx);
-        c[2] = __ldg(p + dy);
-        c[3] = __ldg(p + dx + dy);
-        c[4] = __ldg(p + dz);
-        c[5] = __ldg(p + dx + dz);
-        c[6] = __ldg(p + dy + dz);
-        c[7] = __ldg(p + dx + dy + dz);
+        c[1] = __ldg(p + 1);
+        c[2] = __ldg(q);
+        c[3] = __ldg(q + 1);
+        c[4] = __ldg(r);
+        c[5] = __ldg(r + 1);
+        c[6] = __ldg(t);
+        c[7] = __ldg(t + 1);
     }
-    __device__ __forceinline__ void corners(int a, const Stencil& st, float c[8]) const
+    __device__ __forceinline__ void corners(int comp, const Corner& st, float c[8]) const
     {
-        int dx, dy, dz;
-        const size_t base = corner_base(a % 3, st, dx, dy, dz);
-        load8(a, base, dx, dy, dz, c);
+        load8(comp, corner_base(comp, st), c);
+    }
+    // the corner values and their differences from the snapshot's, side by side
+    __device__ __forceinline__ void corners_diff(int comp, const Corner& st, F2 c[8]) const
+    {
+        float a[8], b[8];
+        const size_t base = corner_base(comp, st);  // the grid and its snapshot share the layout
+        load8(comp, base, a);
+        load8(comp + 3, base, b);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) c[t] = pack2(a[t], a[t] - b[t]);
     }
 };
 
-__device__ __forceinline__ float lerp8(const float c[8], const Stencil& s)
+// Trilinear value of the corners, the two z planes side by side.
+__device__ __forceinline__ float lerp8(const float c[8], const Corner& s)
 {
-    const float b0 = lerpf_ref(lerpf_ref(c[0], c[1], s.fx), lerpf_ref(c[2], c[3], s.fx), s.fy);
-    const float b1 = lerpf_ref(lerpf_ref(c[4], c[5], s.fx), lerpf_ref(c[6], c[7], s.fx), s.fy);
+    const F2 mx = pack2(1.f - s.fx, 1.f - s.fx), fx = pack2(s.fx, s.fx), my = pack2(1.f - s.fy, 1.f - s.fy), fy = pack2(s.fy, s.fy);
+    const F2 y0 = lerp2(pack2(c[0], c[4]), pack2(c[1], c[5]), mx, fx), y1 = lerp2(pack2(c[2], c[6]), pack2(c[3], c[7]), mx, fx);
+    float b0, b1;
+    unpack2(lerp2(y0, y1, my, fy), b0, b1);
     return lerpf_ref(b0, b1, s.fz);
 }
+// ... of both values of each corner.
+__device__ __forceinline__ void lerp8x2(const F2 c[8], const Corner& s, float& first, float& second)
+{
+    const F2 mx = pack2(1.f - s.fx, 1.f - s.fx), fx = pack2(s.fx, s.fx), my = pack2(1.f - s.fy, 1.f - s.fy), fy = pack2(s.fy, s.fy);
+    F2 z[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        z[k] = lerp2(lerp2(c[4 * k], c[4 * k + 1], mx, fx), lerp2(c[4 * k + 2], c[4 * k + 3], mx, fx), my, fy);
+    unpack2(lerp2(z[0], z[1], pack2(1.f - s.fz, 1.f - s.fz), pack2(s.fz, s.fz)), first, second);
+}
 
-// GetBarycentric index pair and fraction of a point along one axis of one staggered grid (stencil() per axis).
+// GetBarycentric index and fraction of a point along one axis of one staggered grid, bary()'s cases by clamping: the
+// position between the first and the last face (NaN: the first), its floor below the last.
 struct AxisFrac {
-    int i, ip;
+    int i;
     float f;
 };
 __device__ __forceinline__ AxisFrac axis_frac(float x, float o, float ih, int size)
 {
+    const float t = fminf(fmaxf((x - o) * ih, 0.f), (float)(size - 1));
+    const float s = fminf(floorf(t), (float)(size - 2));
     AxisFrac a;
-    bary((x - o) * ih, size - 1, a.i, a.f);
-    a.ip = min(a.i + 1, size - 1);
+    a.i = (int)s;
+    a.f = t - s;
     return a;
 }
-__device__ __forceinline__ Stencil stencil_of(const AxisFrac& a, const AxisFrac& b, const AxisFrac& c)
+__device__ __forceinline__ Corner stencil_of(const AxisFrac& a, const AxisFrac& b, const AxisFrac& c)
 {
-    Stencil s;
-    s.i = a.i; s.ip = a.ip; s.fx = a.f;
-    s.j = b.i; s.jp = b.ip; s.fy = b.f;
-    s.k = c.i; s.kp = c.ip; s.fz = c.f;
+    Corner s;
+    s.i = a.i; s.fx = a.f;
+    s.j = b.i; s.fy = b.f;
+    s.k = c.i; s.fz = c.f;
     return s;
 }
 
@@ -82,8 +129,8 @@ __device__ __forceinline__ Stencil stencil_of(const AxisFrac& a, const AxisFrac&
 // xo[1] == zo[1], yo[0] == zo[0], xo[2] == yo[2], and likewise for the FLIP residual origins) and the same size, so
 // their index and fraction are one computation: 6 per point instead of 9.
 __device__ __forceinline__ void stencils3(float x, float y, float z, const float ou[3], const float ov[3],
-                                          const float ow[3], const float ih[3], int nx, int ny, int nz, Stencil& su,
-                                          Stencil& sv, Stencil& sw)
+                                          const float ow[3], const float ih[3], int nx, int ny, int nz, Corner& su,
+                                          Corner& sv, Corner& sw)
 {
     const AxisFrac xf = axis_frac(x, ou[0], ih[0], nx + 1), xc = axis_frac(x, ov[0], ih[0], nx);
     const AxisFrac yf = axis_frac(y, ov[1], ih[1], ny + 1), yc = axis_frac(y, ou[1], ih[1], ny);
@@ -104,92 +151,73 @@ __device__ __forceinline__ void sample_vel(const SceneView& v, const FaceSource&
     const AxisFrac xf = axis_frac(x, v.xo[0], ih[0], nx + 1);
     const AxisFrac yc = axis_frac(y, v.xo[1], ih[1], ny);
     const AxisFrac zc = axis_frac(z, v.xo[2], ih[2], nz);
-    const Stencil su = stencil_of(xf, yc, zc);
+    const Corner su = stencil_of(xf, yc, zc);
     fs.corners(0, su, c);
     out[0] = lerp8(c, su);
     const AxisFrac xc = axis_frac(x, v.yo[0], ih[0], nx);
     const AxisFrac yf = axis_frac(y, v.yo[1], ih[1], ny + 1);
-    const Stencil sv = stencil_of(xc, yf, zc);
+    const Corner sv = stencil_of(xc, yf, zc);
     fs.corners(1, sv, c);
     out[1] = lerp8(c, sv);
     const AxisFrac zf = axis_frac(z, v.zo[2], ih[2], nz + 1);
-    const Stencil sw = stencil_of(xc, yc, zf);
+    const Corner sw = stencil_of(xc, yc, zf);
     fs.corners(2, sw, c);
     out[2] = lerp8(c, sw);
 }
 
 // Trilinear sample of (grid - snapshot) with the reference's Lerp tree (the FLIP residual grid,
-// flip_simulator.cpp:138-150), and, when `plain` is non-null, the grid's own sample at the same stencil from the
-// same face values.
-__device__ __forceinline__ float sample_diff(const FaceSource& fs, int comp, const Stencil& s, float* plain)
+// flip_simulator.cpp:138-150), and of the grid itself at the same stencil from the same face values.
+__device__ __forceinline__ float sample_diff(const FaceSource& fs, int comp, const Corner& s, float& plain)
 {
-    float a[8], b[8], d[8];
-    int dx, dy, dz;
-    const size_t base = fs.corner_base(comp, s, dx, dy, dz);  // the grid and its snapshot share the layout
-    fs.load8(comp, base, dx, dy, dz, a);
-    fs.load8(comp + 3, base, dx, dy, dz, b);
-#pragma unroll
-    for (int t = 0; t < 8; ++t) d[t] = a[t] - b[t];
-    if (plain) *plain = lerp8(a, s);
-    return lerp8(d, s);
+    F2 c[8];
+    fs.corners_diff(comp, s, c);
+    float diff;
+    lerp8x2(c, s, plain, diff);
+    return diff;
 }
 
-// sum_t gradweight_t * face_t for one velocity component (apic_simulator.cpp:311-336), from the stencil's 8 corner
-// values.
-__device__ __forceinline__ void apic_row_vals(const float val[8], const Stencil& s, const float ih[3], float out[3])
+// sum_t gradweight_t * face_t for one velocity component (apic_simulator.cpp:311-336) from the stencil's 8 corner values:
+// per axis the differences of the corners along it, interpolated along the others, over h.  Returns the trilinear value,
+// whose partial sums the rows share.
+__device__ __forceinline__ float apic_row_vals(const float c[8], const Corner& s, const float ih[3], float out[3])
 {
-    const float fx = s.fx, fy = s.fy, fz = s.fz;
-    const float gx[8] = {-ih[0] * (1 - fy) * (1 - fz), ih[0] * (1 - fy) * (1 - fz), (-ih[0]) * fy * (1 - fz),
-                         ih[0] * fy * (1 - fz),        (-ih[0]) * (1 - fy) * fz,   ih[0] * (1 - fy) * fz,
-                         (-ih[0]) * fy * fz,           ih[0] * fy * fz};
-    const float gy[8] = {-ih[1] * (1 - fx) * (1 - fz), fx * (-ih[1]) * (1 - fz), (1 - fx) * ih[1] * (1 - fz),
-                         fx * ih[1] * (1 - fz),        (1 - fx) * (-ih[1]) * fz, fx * (-ih[1]) * fz,
-                         (1 - fx) * ih[1] * fz,        fx * ih[1] * fz};
-    const float gz[8] = {-ih[2] * (1 - fx) * (1 - fy), fx * (1 - fy) * (-ih[2]), (1 - fx) * fy * (-ih[2]),
-                         fx * fy * (-ih[2]),           (1 - fx) * (1 - fy) * ih[2], fx * (1 - fy) * ih[2],
-                         (1 - fx) * fy * ih[2],        fx * fy * ih[2]};
-    float r0 = 0.f, r1 = 0.f, r2 = 0.f;
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-        r0 += gx[t] * val[t];
-        r1 += gy[t] * val[t];
-        r2 += gz[t] * val[t];
-    }
-    out[0] = r0;
-    out[1] = r1;
-    out[2] = r2;
-}
-
-__device__ __forceinline__ void apic_row(const FaceSource& fs, int comp, const Stencil& s, const float ih[3],
-                                         float out[3])
-{
-    float val[8];
-    fs.corners(comp, s, val);
-    apic_row_vals(val, s, ih, out);
+    const F2 mx = pack2(1.f - s.fx, 1.f - s.fx), fx = pack2(s.fx, s.fx), my = pack2(1.f - s.fy, 1.f - s.fy), fy = pack2(s.fy, s.fy);
+    const F2 y0 = lerp2(pack2(c[0], c[4]), pack2(c[1], c[5]), mx, fx), y1 = lerp2(pack2(c[2], c[6]), pack2(c[3], c[7]), mx, fx);
+    float x0, x1;  // along x, lower and upper z plane
+    unpack2(lerp2(pack2(c[1] - c[0], c[5] - c[4]), pack2(c[3] - c[2], c[7] - c[6]), my, fy), x0, x1);
+    float a0, a1, e0, e1, b0, b1;
+    unpack2(y0, a0, a1);
+    unpack2(y1, e0, e1);
+    unpack2(lerp2(y0, y1, my, fy), b0, b1);
+    out[0] = ih[0] * lerpf_ref(x0, x1, s.fz);
+    out[1] = ih[1] * lerpf_ref(e0 - a0, e1 - a1, s.fz);
+    out[2] = ih[2] * (b1 - b0);
+    return lerpf_ref(b0, b1, s.fz);
 }
 
 // APIC: component c's grid sample at the particle (stencil s, the velocity grid's face counts as sizes) and its C row.
 // The row's stencil is taken at the particle clamped by h/2 on the two transverse axes with the CELL counts as sizes;
 // where no clamp moves the particle and its index along the component's own axis is below n - 1 (the two sizes then
 // give the same GetBarycentric result), it is s itself, and the row reuses the sample's 8 corner values.
-__device__ __forceinline__ float apic_component(const SceneView& v, const FaceSource& fs, int c, const Stencil& s,
+__device__ __forceinline__ float apic_component(const SceneView& v, const FaceSource& fs, int c, const Corner& s,
                                                 const float P[3], const float lo[3], const float hi[3], uint64_t p)
 {
     float c8[8];
     fs.corners(c, s, c8);
-    const float pic = lerp8(c8, s);
+    float row[3];
+    const float pic = apic_row_vals(c8, s, v.inv_hf, row);
     float q[3] = {P[0], P[1], P[2]};
 #pragma unroll
     for (int a = 0; a < 3; ++a)
         if (a != c) q[a] = q[a] < lo[a] ? lo[a] : (q[a] > hi[a] ? hi[a] : q[a]);
     const int n_c = c == 0 ? v.g.nx : (c == 1 ? v.g.ny : v.g.nz);
     const int i_c = c == 0 ? s.i : (c == 1 ? s.j : s.k);
-    float row[3];
-    if (q[0] == P[0] && q[1] == P[1] && q[2] == P[2] && i_c <= n_c - 2) {
-        apic_row_vals(c8, s, v.inv_hf, row);
-    } else {
+    if (!(q[0] == P[0] && q[1] == P[1] && q[2] == P[2] && i_c <= n_c - 2)) {
         const float* org = c == 0 ? v.xo : (c == 1 ? v.yo : v.zo);
-        apic_row(fs, c, stencil(q[0], q[1], q[2], org, v.inv_hf, v.g.nx, v.g.ny, v.g.nz), v.inv_hf, row);
+        const Corner t = stencil_of(axis_frac(q[0], org[0], v.inv_hf[0], v.g.nx), axis_frac(q[1], org[1], v.inv_hf[1], v.g.ny),
+                                    axis_frac(q[2], org[2], v.inv_hf[2], v.g.nz));
+        fs.corners(c, t, c8);
+        apic_row_vals(c8, t, v.inv_hf, row);
     }
     v.c[3 * c][p] = row[0];
     v.c[3 * c + 1][p] = row[1];
@@ -230,12 +258,11 @@ __device__ __forceinline__ void g2p_particle(const SceneView& v, const G2PArgs& 
     bool have_pic = false;
     if (G2P) {
         if (SOLVER == FE_SOLVER_FLIP) {
-            Stencil su, sv, sw;
+            Corner su, sv, sw;
             stencils3(x, y, z, v.rxo, v.ryo, v.rzo, v.inv_hf, nx, ny, nz, su, sv, sw);
             const bool share = g.same_origins && v.blend > 0.f;
-            float flip[3] = {v.vx[p] + sample_diff(fs, 0, su, share ? &pic[0] : nullptr),
-                             v.vy[p] + sample_diff(fs, 1, sv, share ? &pic[1] : nullptr),
-                             v.vz[p] + sample_diff(fs, 2, sw, share ? &pic[2] : nullptr)};
+            float flip[3] = {v.vx[p] + sample_diff(fs, 0, su, pic[0]), v.vy[p] + sample_diff(fs, 1, sv, pic[1]),
+                             v.vz[p] + sample_diff(fs, 2, sw, pic[2])};
             if (v.blend > 0.f) {
                 if (!share) sample_vel(v, fs, x, y, z, pic);
                 have_pic = true;
@@ -302,8 +329,10 @@ __device__ __forceinline__ FaceSource global_source(const SceneView& v, const G2
 }
 
 // One thread per particle over the sorted arrays: neighbouring threads hold neighbouring particles, so the face
-// gathers hit L1/L2.  (A variant staging each tile's faces in shared memory, 13^3 per array, measured slower:
-// 260 us against 183 us per launch at 128^3 FLIP.)
+// gathers hit L1/L2.  Bound by the L1's address lookups (86 % at 128^3 FLIP) and issue: 149 us there and 1596 us at 256^3
+// APIC (32 M particles) with the indexes of clamped pairs, an address per corner and one sample at a time, 135 and 1225 with
+// rows of two faces and packed interpolation (968 against 648 instructions a particle).  The faces of half a tile in shared
+// memory (12 x 12 x 8 per component, read by the half tile's particles) took 136 and 1080, but 12 us more at 32^3.
 template <int SOLVER, bool G2P, bool MOVE>
 __global__ void __launch_bounds__(256, 4) k_g2p(SceneView v, G2PArgs g)
 {
