@@ -12,9 +12,10 @@
 // use every crossed edge (and every inside corner of a square), so all items around a key create or look it up,
 // and the one that creates it is the first of them in sweep order -- a closed-form function of the key (along
 // each axis across the key, the item with the smaller index when both exist).  So:
-//   k_mc_count  per item: the case byte, its triangles and the keys it creates;
+//   k_mc_count_cubes, k_mc_count_caps  per item: the case byte, its triangles and the keys it creates, and a list of
+//               the items with triangles;
 //   two exclusive scans over items give each item its first vertex and first triangle;
-//   k_mc_emit   per item with triangles: creates its keys' vertices (position, normal) at base + rank in its
+//   k_mc_emit   per listed item: creates its keys' vertices (position, normal) at base + rank in its
 //               own use order, and resolves the other keys to the creating item's base + rank, recomputed from
 //               that item's case byte.
 // The arithmetic is the reference's, operation by operation in FP64 with explicit round-to-nearest intrinsics (no
@@ -129,16 +130,7 @@ __device__ __forceinline__ bool creates(const int off[3], const int c[3], int sk
     return true;
 }
 
-// Case byte and the packed triangle list of an item.
-__device__ __forceinline__ int cube_case(const McGrid& g, int i, int j, int k)
-{
-    int cfg = 0;
-#pragma unroll
-    for (int v = 0; v < 8; ++v)
-        if (sdf_at(g, i + c_corner_off[v][0], j + c_corner_off[v][1], k + c_corner_off[v][2]) <= 0.0) cfg |= 1 << v;
-    return cfg;
-}
-
+// Case bits of a cap square.
 __device__ __forceinline__ int cap_case(const McGrid& g, int side, const int c[3])
 {
     int cfg = 0;
@@ -186,28 +178,87 @@ __device__ int creation_rank(int kind, int side, const int c[3], int cfg, int ta
     return -1;
 }
 
-__global__ void k_mc_count(McGrid g, uint64_t items, uint8_t* __restrict__ cfg_out, uint32_t* __restrict__ nvert,
-                           uint32_t* __restrict__ ntri)
+// Case byte, vertices created and triangles of an item; items with triangles are listed (in any order: the scans give
+// each its place).  All lanes of the warp take part; `on`: the lane has an item.
+__device__ __forceinline__ void count_item(const McGrid& g, bool on, uint64_t t, const Item& it, int cfg,
+                                           uint8_t* __restrict__ cfg_out, uint32_t* __restrict__ nvert,
+                                           uint32_t* __restrict__ ntri, uint32_t* __restrict__ active)
 {
-    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < items; t += (uint64_t)gridDim.x * blockDim.x) {
-        const Item it = decode(g, t);
-        const int cfg = it.kind == 0 ? cube_case(g, it.c[0], it.c[1], it.c[2]) : cap_case(g, it.side, it.c);
-        cfg_out[t] = (uint8_t)cfg;
+    int created = 0, nt = 0;
+    if (on && cfg != 0 && !(it.kind == 0 && cfg == 255)) {
         const unsigned long long cs = it.kind == 0 ? c_case3[cfg] : c_case2[cfg];
-        const int nt = (int)(cs >> 60);
+        nt = (int)(cs >> 60);
         unsigned used = 0u;
         for (int q = 0; q < 3 * nt; ++q) used |= 1u << ((cs >> (4 * q)) & 15);
         const int skip = skip_axis_of(it.kind, it.side);
-        int created = 0;
         for (int q = 0; q < 12; ++q) {
             if (!((used >> q) & 1u)) continue;
             int off[3];
             key_off(it.kind, it.side, q, off);
             if (creates(off, it.c, skip)) ++created;
         }
+    }
+    if (on) {
+        cfg_out[t] = (uint8_t)cfg;
         nvert[t] = (uint32_t)created;
         ntri[t] = (uint32_t)nt;
     }
+    const unsigned some = __ballot_sync(0xffffffffu, nt > 0);
+    if (some) {
+        const int lane = (int)threadIdx.x & 31;
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(active, (uint32_t)__popc(some));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (nt > 0) active[1 + base + __popc(some & ((1u << lane) - 1u))] = (uint32_t)t;
+    }
+}
+
+// The cubes of 32 x 1 x 32 cells a block.  The items run along z and the SDF along x, so a block turns the signs of its
+// nodes in shared memory: both sides then move in whole lines (with a thread per item reading its 8 nodes 75 us at 128^3).
+constexpr int kMcW = 32;
+__global__ void __launch_bounds__(256) k_mc_count_cubes(McGrid g, uint8_t* __restrict__ cfg_out, uint32_t* __restrict__ nvert,
+                                                        uint32_t* __restrict__ ntri, uint32_t* __restrict__ active)
+{
+    __shared__ uint8_t in[2][kMcW + 1][kMcW + 4];  // y, z, x: the node is inside
+    const int i0 = (int)blockIdx.x * kMcW, j = (int)blockIdx.y, k0 = (int)blockIdx.z * kMcW;
+    for (int q = (int)threadIdx.x; q < 2 * (kMcW + 1) * (kMcW + 1); q += 256) {
+        const int i = q % (kMcW + 1), k = q / (kMcW + 1) % (kMcW + 1), y = q / ((kMcW + 1) * (kMcW + 1));
+        if (i0 + i < g.n[0] && k0 + k < g.n[2]) in[y][k][i] = sdf_at(g, i0 + i, j + y, k0 + k) <= 0.0 ? 1 : 0;
+    }
+    __syncthreads();
+    const int k = (int)threadIdx.x & 31;
+    for (int i = (int)threadIdx.x >> 5; i < kMcW; i += 8) {
+        const bool on = i0 + i < g.n[0] - 1 && k0 + k < g.n[2] - 1;
+        Item it;
+        it.kind = 0;
+        it.side = 0;
+        it.c[0] = i0 + i;
+        it.c[1] = j;
+        it.c[2] = k0 + k;
+        int cfg = 0;
+        if (on)
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+                constexpr int off[8][3] = FE_MC_CORNER_OFFSETS;
+                cfg |= in[off[v][1]][k + off[v][2]][i + off[v][0]] << v;
+            }
+        count_item(g, on, on ? encode_cube(g, it.c[0], it.c[1], it.c[2]) : 0, it, cfg, cfg_out, nvert, ntri, active);
+    }
+}
+// The cap squares, an item a thread.
+__global__ void __launch_bounds__(256) k_mc_count_caps(McGrid g, uint64_t items, uint8_t* __restrict__ cfg_out,
+                                                       uint32_t* __restrict__ nvert, uint32_t* __restrict__ ntri,
+                                                       uint32_t* __restrict__ active)
+{
+    const uint64_t t = g.cubes + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    const bool on = t < items;
+    Item it{};
+    int cfg = 0;
+    if (on) {
+        it = decode(g, t);
+        cfg = cap_case(g, it.side, it.c);
+    }
+    count_item(g, on, t, it, cfg, cfg_out, nvert, ntri, active);
 }
 
 __device__ __forceinline__ double dm(double a, double b) { return __dmul_rn(a, b); }
@@ -287,13 +338,18 @@ __device__ void cap_vertex(const McGrid& g, int side, const int c[3], int q, dou
     for (int d = 0; d < 3; ++d) p[d] = da(dm(w0, grid_pos(g, d, na[d])), dm(alpha, grid_pos(g, d, nb[d])));
 }
 
-__global__ void k_mc_emit(McGrid g, uint64_t items, const uint8_t* __restrict__ cfgs, const uint32_t* __restrict__ vbase,
-                          const uint32_t* __restrict__ tbase, double* __restrict__ V, double* __restrict__ N,
-                          int64_t* __restrict__ T)
+// One listed item a thread: bound by the latency of its chain of FP64 divisions and lookups, so small blocks spread the list
+// over the SMs.  (Over all items, most of them without triangles, 126 us at 128^3.)
+constexpr int kMcEmit = 64;
+__global__ void __launch_bounds__(kMcEmit) k_mc_emit(McGrid g, const uint32_t* __restrict__ active, uint32_t n_active,
+                                                     const uint8_t* __restrict__ cfgs, const uint32_t* __restrict__ vbase,
+                                                     const uint32_t* __restrict__ tbase, double* __restrict__ V,
+                                                     double* __restrict__ N, int64_t* __restrict__ T)
 {
-    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < items; t += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t e = blockIdx.x * (uint32_t)kMcEmit + threadIdx.x;
+    if (e < n_active) {
+        const uint64_t t = active[e];
         const uint32_t tb = tbase[t];
-        if (tbase[t + 1] == tb) continue;
         const Item it = decode(g, t);
         const int cfg = cfgs[t];
         const unsigned long long cs = it.kind == 0 ? c_case3[cfg] : c_case2[cfg];
@@ -366,8 +422,8 @@ size_t mc_items(int nx, int ny, int nz)
     return mx * my * mz + 2 * (my * mx + mz * my + mz * mx);
 }
 
-cudaError_t launch_mc_count(const SceneView& v, const double* sdf, uint8_t* cfg, uint32_t* nvert, uint32_t* ntri,
-                            cudaStream_t st)
+namespace {
+McGrid mc_grid(const SceneView& v, const double* sdf)
 {
     McGrid g;
     g.n[0] = v.g.nx; g.n[1] = v.g.ny; g.n[2] = v.g.nz;
@@ -378,28 +434,30 @@ cudaError_t launch_mc_count(const SceneView& v, const double* sdf, uint8_t* cfg,
     g.part0[0] = g.cubes;
     g.part0[1] = g.part0[0] + 2 * my * mx;
     g.part0[2] = g.part0[1] + 2 * mz * my;
-    const uint64_t items = g.part0[2] + 2 * mz * mx;
-    const unsigned blocks = (unsigned)std::min<uint64_t>((items + 255) / 256, 148 * 16);
-    k_mc_count<<<blocks, 256, 0, st>>>(g, items, cfg, nvert, ntri);
-    count_launch();
+    return g;
+}
+}  // namespace
+
+cudaError_t launch_mc_count(const SceneView& v, const double* sdf, uint8_t* cfg, uint32_t* nvert, uint32_t* ntri,
+                            uint32_t* active, cudaStream_t st)
+{
+    const McGrid g = mc_grid(v, sdf);
+    const uint64_t items = mc_items(g.n[0], g.n[1], g.n[2]);
+    cudaError_t e = cudaMemsetAsync(active, 0, sizeof(uint32_t), st);
+    if (e != cudaSuccess) return e;
+    k_mc_count_cubes<<<dim3((unsigned)((g.n[0] - 2) / kMcW + 1), (unsigned)(g.n[1] - 1), (unsigned)((g.n[2] - 2) / kMcW + 1)), 256,
+                       0, st>>>(g, cfg, nvert, ntri, active);
+    k_mc_count_caps<<<(unsigned)((items - g.cubes + 255) / 256), 256, 0, st>>>(g, items, cfg, nvert, ntri, active);
+    count_launch(2);
     return cudaGetLastError();
 }
 
-cudaError_t launch_mc_emit(const SceneView& v, const double* sdf, const uint8_t* cfg, const uint32_t* vbase,
-                           const uint32_t* tbase, double* V, double* N, int64_t* T, cudaStream_t st)
+cudaError_t launch_mc_emit(const SceneView& v, const double* sdf, const uint32_t* active, uint32_t n_active, const uint8_t* cfg,
+                           const uint32_t* vbase, const uint32_t* tbase, double* V, double* N, int64_t* T, cudaStream_t st)
 {
-    McGrid g;
-    g.n[0] = v.g.nx; g.n[1] = v.g.ny; g.n[2] = v.g.nz;
-    for (int a = 0; a < 3; ++a) { g.o[a] = v.sdf_origin[a]; g.h[a] = v.h[a]; }
-    g.sdf = sdf;
-    const uint64_t mx = g.n[0] - 1, my = g.n[1] - 1, mz = g.n[2] - 1;
-    g.cubes = mx * my * mz;
-    g.part0[0] = g.cubes;
-    g.part0[1] = g.part0[0] + 2 * my * mx;
-    g.part0[2] = g.part0[1] + 2 * mz * my;
-    const uint64_t items = g.part0[2] + 2 * mz * mx;
-    const unsigned blocks = (unsigned)std::min<uint64_t>((items + 255) / 256, 148 * 16);
-    k_mc_emit<<<blocks, 256, 0, st>>>(g, items, cfg, vbase, tbase, V, N, T);
+    if (n_active == 0) return cudaSuccess;
+    k_mc_emit<<<(n_active + kMcEmit - 1) / kMcEmit, kMcEmit, 0, st>>>(mc_grid(v, sdf), active + 1, n_active, cfg, vbase, tbase, V, N,
+                                                                      T);
     count_launch();
     return cudaGetLastError();
 }
