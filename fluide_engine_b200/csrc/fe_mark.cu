@@ -452,16 +452,16 @@ __global__ void k_node_values(double* node, size_t nc, double band, double radiu
 // The same node values from particles that are grouped by cell, gathered per node: no atomics, and nearly every node
 // inside the fluid is decided by its own cell, because a particle nearer than half a cell is nearer than any of another
 // cell.  A block takes a tile's nodes.  Nodes whose own cell doesn't decide are listed, so that warps are full again, and
-// walk the occupied cells up to two away (the band is at most 2.5 cells wide, see node_reach), nearer rows first; a row or
-// cell is skipped when its nearest point is further away than the smallest distance so far.  The bucket test of the
-// reference's search is made for the nearest particle alone.  Where it fails (the nearest one doesn't count), or a cell holds
-// too many particles for one thread, a warp searches all cells with the test for each particle.  `order` (optional) gives
-// the particle of each slot of the cells' runs.
+// walk the occupied cells up to two away (the band is at most 2.5 cells wide, see node_reach), nearer ones first; a
+// cell is skipped when its nearest point is further away than the smallest distance so far.  Where a cell holds too many
+// particles for one thread, a warp searches all cells.  `order` (optional) gives the particle of each slot of the cells'
+// runs.
 //
 // Bound by the latency of the listed nodes' searches (a lone particle has some 80 nodes search for it).  Against the scatter
 // over particles below, which tests 64 nodes a particle and reads 21 of them: 4 M particles at 128^3 (FLIP dam with spray,
-// unsorted) 512 us against 208, and 50 for grouping them; 0.5 M sorted ones at 64^3 92 against 58.  With one walk over the
-// rows instead of the groups of bits 321 and 82, with a warp per listed node 630 and 160.
+// unsorted) 512 us against 183, and 50 for grouping them; 0.5 M sorted ones at 64^3 92 against 50.  With a warp per listed
+// node 630 and 160, with one walk over the rows instead of the groups of bits 321 and 82, with the bucket test for the nearest
+// particle alone and a warp's search where it fails 210 and 58; four lanes a listed node gave nothing.
 //
 // The 125 cells around a node come in five groups, nearer ones first: the 27 that touch the node's cell, those two away along
 // x in the same rows, then the 16 rows around (6, 6 and 4 of 5 cells).  A thread collects a group's occupied cells as bits
@@ -471,7 +471,9 @@ struct NodeReach {
     double near2[kNodeCells];         // squared distance from a node to the nearest point of the cell
     double group2[kNodeGroups];       // the smallest of the group
     uint32_t valid[kNodeGroups];      // cells that reach into the band
+    int8_t span[25];                  // of a row, (dy + 2) + 5 (dz + 2): cells at most so far along x do (-1: none)
     double own2;                      // squared distance up to which the node's own cell decides
+    double safe2;                     // ... and below which a particle is in a bucket that the node's search visits
 };
 __host__ __device__ constexpr int node_group_first(int w) { return w == 0 ? 0 : (w == 1 ? 27 : 45 + 30 * (w - 2)); }
 // Rows around a node, (dy + 2) + 5 (dz + 2): the 9 that touch its cell's row, then the 16 around, nearer ones first.
@@ -481,7 +483,7 @@ __host__ __device__ constexpr int node_row(int r)
     return rows[r];
 }
 // Offset of the cell of bit `bit` of group `w`.
-__host__ __device__ inline void node_cell(int w, int bit, int d[3])
+__host__ __device__ constexpr void node_cell(int w, int bit, int d[3])
 {
     const int width = w == 0 ? 3 : (w == 1 ? 2 : 5);
     const int row = node_row(w < 2 ? bit / width : 9 + 6 * (w - 2) + bit / width), x = bit % width;
@@ -490,14 +492,33 @@ __host__ __device__ inline void node_cell(int w, int bit, int d[3])
     d[2] = row / 5 - 2;
 }
 
+// Offsets of the cells in a block's halo, group after group.
+struct NodeOffsets {
+    int16_t at[kNodeCells];
+};
+
 // A block takes half a tile: 256 nodes, and the cells up to two around them.
 constexpr int kNodeLayers = FE_TILE / 2;
 constexpr int kNodeThreads = FE_TILE * FE_TILE * kNodeLayers;
 constexpr int kNodeHalo = FE_TILE + 4, kNodeHaloZ = kNodeLayers + 4;
 constexpr uint32_t kNodeLaneCap = 32;  // particles a thread tests for one cell; fuller cells are spread over a warp
+constexpr NodeOffsets make_node_offsets()
+{
+    NodeOffsets t{};
+    int n = 0;
+    for (int w = 0; w < kNodeGroups; ++w)
+        for (int bit = 0; n < (w + 1 < kNodeGroups ? node_group_first(w + 1) : kNodeCells); ++bit) {
+            int d[3] = {0, 0, 0};
+            node_cell(w, bit, d);
+            t.at[n++] = (int16_t)(d[0] + kNodeHalo * (d[1] + kNodeHalo * d[2]));
+        }
+    return t;
+}
+__device__ const NodeOffsets g_node_offsets = make_node_offsets();
 struct NodeShared {
     uint32_t start[kNodeHalo * kNodeHalo * kNodeHaloZ], count[kNodeHalo * kNodeHalo * kNodeHaloZ];
     uint16_t row[kNodeHalo * kNodeHaloZ];  // occupied cells of a row, a bit each
+    uint8_t near[FE_TILE * kNodeLayers];   // nodes of a row with an occupied cell that reaches into their band
     uint16_t list[kNodeThreads];           // nodes to search, a thread each
     uint16_t hard[kNodeThreads];           // ... a warp each
     double near2[kNodeCells];
@@ -540,12 +561,8 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
             sh.count[q] = end - beg;
         }
         if (threadIdx.x < kNodeCells) {
-            const int c = (int)threadIdx.x;
-            const int w = c < 27 ? 0 : (c < 45 ? 1 : 2 + (c - 45) / 30);
-            int d[3];
-            node_cell(w, c - node_group_first(w), d);
-            sh.near2[c] = reach.near2[c];
-            sh.cell[c] = (int16_t)(d[0] + kNodeHalo * (d[1] + kNodeHalo * d[2]));
+            sh.near2[threadIdx.x] = reach.near2[threadIdx.x];
+            sh.cell[threadIdx.x] = g_node_offsets.at[threadIdx.x];
         }
         if (threadIdx.x == 0) sh.n = sh.nhard = 0;
     }
@@ -556,6 +573,20 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
             for (int i = 0; i < kNodeHalo; ++i) bits |= sh.count[r * kNodeHalo + i] ? 1u << i : 0u;
             sh.row[r] = (uint16_t)bits;
         }
+    __syncthreads();
+    if (occupied && threadIdx.x < FE_TILE * kNodeLayers) {
+        const uint16_t* row = sh.row + (threadIdx.x & 7) + kNodeHalo * (threadIdx.x >> 3);
+        unsigned bits = 0;
+#pragma unroll
+        for (int b = 0; b < 25; ++b) {
+            const unsigned x = row[b % 5 + kNodeHalo * (b / 5)];  // bit i + 2: the cell of node i
+            const int span = reach.span[b];
+            if (span >= 0) bits |= x >> 2;
+            if (span >= 1) bits |= (x >> 1) | (x >> 3);
+            if (span >= 2) bits |= x | (x >> 4);
+        }
+        sh.near[threadIdx.x] = (uint8_t)bits;
+    }
     __syncthreads();
     // occupied cells of group w around local node (lx, ly, lz) that reach into the band
     auto group = [&](int w, int lx, int ly, int lz) {
@@ -581,48 +612,31 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
         return m & reach.valid[w];
     };
 
-    const double none = __longlong_as_double(0x7ff0000000000000ll);  // infinite: no particle within the band
-    auto value = [&](double best) { return __dsub_rn(best == none ? v.band : fmin(__dsqrt_rn(best), v.band), v.radius); };
+    auto value = [&](double best) { return __dsub_rn(best > R2 ? v.band : fmin(__dsqrt_rn(best), v.band), v.radius); };
     auto bucket_ok = [&](double X, double Y, double Z, int i, int j, int k) {
         return visited(v, bucket_fast(X, v.bucket, inv_bucket), bucket_fast(Y, v.bucket, inv_bucket),
                        bucket_fast(Z, v.bucket, inv_bucket), i, j, k);
     };
-    // the nearest of the particles in slots [s, s + n) by the reference's squared distance, if nearer than best
-    auto nearest = [&](uint32_t s, uint32_t n, double qx, double qy, double qz, double& best, uint32_t& arg) {
+    // the nearest of the particles in slots [s, s + n) by the reference's squared distance, if nearer than best; the
+    // buckets decide about particles more than half a bucket away only
+    auto nearest = [&](uint32_t s, uint32_t n, int i, int j, int k, double qx, double qy, double qz, double& best) {
         constexpr int B = 4;
         for (uint32_t e = 0; e < n; e += B) {
-            uint32_t p[B];
             float x[B], y[B], z[B];
 #pragma unroll
             for (int b = 0; b < B; ++b) {
                 const uint32_t at = s + min(e + b, n - 1);
-                p[b] = ORDER ? __ldg(order + at) : at;
-            }
-#pragma unroll
-            for (int b = 0; b < B; ++b) {
-                x[b] = __ldg(v.px + p[b]);
-                y[b] = __ldg(v.py + p[b]);
-                z[b] = __ldg(v.pz + p[b]);
+                const uint32_t p = ORDER ? __ldg(order + at) : at;
+                x[b] = __ldg(v.px + p);
+                y[b] = __ldg(v.py + p);
+                z[b] = __ldg(v.pz + p);
             }
 #pragma unroll
             for (int b = 0; b < B; ++b) {
                 const double d2 = dist2_ref((double)x[b], (double)y[b], (double)z[b], qx, qy, qz);
-                if (d2 < best) {
-                    best = d2;
-                    arg = p[b];
-                }
+                if (d2 < best && (d2 < reach.safe2 || bucket_ok((double)x[b], (double)y[b], (double)z[b], i, j, k))) best = d2;
             }
         }
-    };
-    const uint32_t nobody = 0xffffffffu;
-    // a node's value from the nearest particle found, or the node goes to the warps
-    auto finish = [&](int t, int i, int j, int k, double best, uint32_t arg) {
-        if (arg == nobody) best = none;
-        else if (!bucket_ok((double)__ldg(v.px + arg), (double)__ldg(v.py + arg), (double)__ldg(v.pz + arg), i, j, k)) {
-            sh.hard[atomicAdd(&sh.nhard, 1)] = (uint16_t)t;
-            return;
-        }
-        out[idx3(i, j, k, nx, ny)] = value(best);
     };
     const double beyond = __longlong_as_double(__double_as_longlong(R2) + 1);  // the next double: best <= R2 counts
 
@@ -632,21 +646,15 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
         const int i = x0 + lx, j = y0 + ly, k = z0 + lz;
         if (i < nx && j < ny && k < nz) {
             double best = beyond;
-            uint32_t arg = nobody;
             bool more = false;
             if (occupied) {
                 const int q = lx + 2 + kNodeHalo * (ly + 2 + kNodeHalo * (lz + 2));
                 const uint32_t n = sh.count[q];
-                if (n > 0 && n <= kNodeLaneCap) nearest(sh.start[q], n, v.q_pos[0][i], v.q_pos[1][j], v.q_pos[2][k], best, arg);
-                if (!(best <= reach.own2)) {
-                    unsigned m = 0;
-#pragma unroll
-                    for (int w = 0; w < kNodeGroups; ++w) m |= group(w, lx, ly, lz);
-                    more = m != 0;
-                }
+                if (n > 0 && n <= kNodeLaneCap) nearest(sh.start[q], n, i, j, k, v.q_pos[0][i], v.q_pos[1][j], v.q_pos[2][k], best);
+                more = !(best <= reach.own2) && ((sh.near[t >> 3] >> lx) & 1u);
             }
             if (more) sh.list[atomicAdd(&sh.n, 1)] = (uint16_t)t;
-            else finish(t, i, j, k, best, arg);
+            else out[idx3(i, j, k, nx, ny)] = value(best);
         }
     }
     if (!occupied) return;
@@ -659,7 +667,6 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
         const int q0 = lx + 2 + kNodeHalo * (ly + 2 + kNodeHalo * (lz + 2));
         const double qx = v.q_pos[0][i], qy = v.q_pos[1][j], qz = v.q_pos[2][k];
         double best = beyond;
-        uint32_t arg = nobody;
         bool full = false;
         for (int w = 0; w < kNodeGroups; ++w) {
             if (!(reach.group2[w] < best)) continue;
@@ -669,12 +676,12 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
                 if (!(sh.near2[c] < best)) continue;
                 const int q = q0 + sh.cell[c];
                 const uint32_t n = sh.count[q];
-                if (n <= kNodeLaneCap) nearest(sh.start[q], n, qx, qy, qz, best, arg);
+                if (n <= kNodeLaneCap) nearest(sh.start[q], n, i, j, k, qx, qy, qz, best);
                 else full = true;
             }
         }
         if (full) sh.hard[atomicAdd(&sh.nhard, 1)] = (uint16_t)t;
-        else finish(t, i, j, k, best, arg);
+        else out[idx3(i, j, k, nx, ny)] = value(best);
     }
     __syncthreads();
 
@@ -683,7 +690,7 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
         const uint32_t p = ORDER ? __ldg(order + s) : s;
         const double X = (double)__ldg(v.px + p), Y = (double)__ldg(v.py + p), Z = (double)__ldg(v.pz + p);
         const double d2 = dist2_ref(X, Y, Z, qx, qy, qz);
-        if (d2 < best && d2 <= R2 && bucket_ok(X, Y, Z, i, j, k)) best = d2;
+        if (d2 < best && (d2 < reach.safe2 || bucket_ok(X, Y, Z, i, j, k))) best = d2;
     };
     const int lane = (int)threadIdx.x & 31;
     for (int e = (int)threadIdx.x >> 5; e < sh.nhard; e += kNodeThreads >> 5) {
@@ -691,7 +698,7 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
         const int lx = t & 7, ly = (t >> 3) & 7, lz = t >> 6;
         const int i = x0 + lx, j = y0 + ly, k = z0 + lz;
         const double qx = v.q_pos[0][i], qy = v.q_pos[1][j], qz = v.q_pos[2][k];
-        double best = none;
+        double best = beyond;
         for (int first = 0; first < kNodeCells; first += 32) {  // each lane its cell
             const int c = first + lane;
             uint32_t s = 0, n = 0;
@@ -838,7 +845,9 @@ static bool node_reach(const SceneView& v, NodeReach& r)
     const double R2 = v.band * v.band;
     bool ok = true;
     double near2[3][3];
+    for (int8_t& span : r.span) span = -1;
     r.own2 = HUGE_VAL;
+    r.safe2 = (1.0 - 1e-6) * (0.25 * v.bucket * v.bucket);
     for (int a = 0; a < 3; ++a) {
         const double delta = 1e-6 * (std::fabs(v.origin[a]) + 4.0 * v.size[a]);
         for (int d = 0; d < 3; ++d) {
@@ -857,7 +866,11 @@ static bool node_reach(const SceneView& v, NodeReach& r)
             node_cell(w, c - first, d);
             r.near2[c] = near2[0][std::abs(d[0])] + near2[1][std::abs(d[1])] + near2[2][std::abs(d[2])];
             r.group2[w] = std::min(r.group2[w], r.near2[c]);
-            if (r.near2[c] <= R2) r.valid[w] |= 1u << (c - first);
+            if (r.near2[c] <= R2) {
+                r.valid[w] |= 1u << (c - first);
+                int8_t& span = r.span[(d[1] + 2) + 5 * (d[2] + 2)];
+                span = std::max<int8_t>(span, (int8_t)std::abs(d[0]));
+            }
         }
     }
     return ok;

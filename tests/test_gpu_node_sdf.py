@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 fe = pytest.importorskip("fluide_engine_b200")
 
-GRIDS = [((16, 16, 16), (1, 1, 1), (0, 0, 0)), ((9, 17, 7), (9 / 16, 17 / 16, 7 / 16), (0, 0, 0)),
+GRIDS = [((16, 16, 16), (1, 1, 1), (0, 0, 0)), ((34, 6, 66), (34 / 32, 6 / 32, 66 / 32), (0, 0, 0)), ((9, 17, 7), (9 / 16, 17 / 16, 7 / 16), (0, 0, 0)),
          ((24, 8, 25), (0.96, 0.32, 1.0), (0, 0, 0)), ((12, 20, 10), (1, 1, 1), (0, 0, 0)),
          ((10, 14, 12), (1, 1.4, 1.2), (-0.5, 0.25, 1.0)), ((2, 3, 2), (2 / 16, 3 / 16, 2 / 16), (0, 0, 0))]
 
