@@ -136,17 +136,16 @@ def mg_coarse_cells(n):
 
 
 def uses_multigrid(n, pressure_solver):
-    return pressure_solver == "mgpcg" or (pressure_solver == "auto" and n ** 3 >= (1 << 15))
+    return pressure_solver == "mgpcg" or (pressure_solver == "auto" and n ** 3 >= (1 << 10))
 
 
 def solver_alg_bytes(fluid, its, refs, n, multigrid):
     """Algorithmic bytes of one pressure solve (numpy arrays per substep).  Plain CG: 41 B per FLUID cell per
-    inner iteration.  Multigrid-preconditioned CG: 68 B per FLUID cell per inner iteration over the five
-    level-0 passes (update + pre-smoothing residual 28, restriction read 4, pre-smoothed correction 8,
-    post-smoothing 12, search direction 16) plus 30 B per cell of every coarser level (residual, restriction,
-    correction, smoothing).  Both: 45 B per FLUID cell per FP64 residual pass (refinements + 1)."""
+    inner iteration.  Multigrid-preconditioned CG: 59 B per FLUID cell per inner iteration over the three
+    level-0 passes (update, sweeps and residual 29, correction and sweeps 13, search direction 17) plus 40 B per cell
+    of every coarser level (right-hand side, sweeps and residual, correction and sweeps); halos not counted.  Both: 45 B per FLUID cell per FP64 residual pass (refinements + 1)."""
     if multigrid:
-        return fluid * (its * 68.0 + (refs + 1.0) * 45.0) + its * 30.0 * mg_coarse_cells(n)
+        return fluid * (its * 59.0 + (refs + 1.0) * 45.0) + its * 40.0 * mg_coarse_cells(n)
     return fluid * (its * 41.0 + (refs + 1.0) * 45.0)
 
 
@@ -833,7 +832,7 @@ def main():
     ap.add_argument("--cg-inner-tol", type=float, default=0.0,
                     help="inner FP32 CG residual reduction per refinement (0: the solver's default)")
     ap.add_argument("--pressure-solver", default="auto", choices=["auto", "mgpcg", "cg"],
-                    help="inner pressure solver: auto (multigrid-preconditioned CG from 2^15 cells, plain CG below), "
+                    help="inner pressure solver: auto (multigrid-preconditioned CG from 2^10 cells, plain CG below), "
                          "mgpcg or cg")
     ap.add_argument("--workload", default="single", choices=["single", "batched", "served", "pool256"])
     ap.add_argument("--surface", action="store_true",
@@ -933,7 +932,7 @@ def main():
     fluid = np.array([s["fluid_cells"] for s in stats], dtype=np.float64)
     its = np.array([s["cg_iterations"] for s in stats], dtype=np.float64)
     refs = np.array([s["refinements"] for s in stats], dtype=np.float64)
-    multigrid = uses_multigrid(n, args.pressure_solver) and not args.collider  # collider scenes use the plain CG
+    multigrid = uses_multigrid(n, args.pressure_solver)
     alg_bytes = solver_alg_bytes(fluid, its, refs, n, multigrid)  # per launch
     peak, peak_kind = peaks()
     achieved = alg_bytes.sum() / (cg_ms.sum() / 1e3) / 1e9
@@ -1007,9 +1006,10 @@ def main():
                          "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
                          "algorithmic_bytes_per_launch": float(alg_bytes.mean()),
-                         "note": ("algorithmic bytes = FLUID cells x (68 B x inner iterations + 45 B x FP64 residual "
-                                  "passes) + 30 B x coarse-level cells x inner iterations; the solve is bound by its "
-                                  "grid barriers (about 14 per inner iteration), not by bandwidth: its working set "
+                         "note": ("algorithmic bytes = FLUID cells x (59 B x inner iterations + 45 B x FP64 residual "
+                                  "passes) + 40 B x coarse-level cells x inner iterations; the solve is bound by its "
+                                  "grid barriers (10 per inner iteration) and the passes between them, not by "
+                                  "bandwidth: its working set "
                                   "is L2-resident at 128^3" if multigrid else
                                   "algorithmic bytes = fluid cells x (41 B x inner iterations + 45 B x FP64 residual "
                                   "passes); at 128^3 the CG working set is L2-resident")},

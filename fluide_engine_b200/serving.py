@@ -49,7 +49,7 @@ def scene_bytes(n, particles, solver):
     cells = n ** 3
     faces = 3 * (n + 1) * n * n
     grid = faces * (5 * 4 + 3) + cells * (1 + 8 + 8 + 9 * 4 + 4 + 4 + 4) + (cells // 512 + 1) * 512 * 8
-    grid += cells * 13 // 7  # multigrid levels: mask + residual + correction + scratch per coarse cell (cells / 7)
+    grid += cells * 16 // 7  # multigrid levels: 1 / D + residual + correction + scratch per coarse cell (cells / 7)
     per_particle = 2 * (7 + (9 if solver == _abi.APIC else 0)) * 4 + 3 * 4 + 9 * 4 + 4
     return grid + particles * per_particle
 

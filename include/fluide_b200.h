@@ -65,8 +65,8 @@ typedef struct {
  * refinement; they differ in how many inner iterations that takes.  The reference uses unpreconditioned CG
  * (linear_system/conjugate_gradient_solver.cpp:14-55). */
 typedef enum {
-    FE_PRESSURE_AUTO = 0,    /* default: MGPCG for grids of 2^15 cells (32^3) or more, CG below (faster there) */
-    FE_PRESSURE_MGPCG = 1,   /* CG preconditioned by one multigrid V-cycle: 10-25 inner iterations, 4 L - 2 barriers each */
+    FE_PRESSURE_AUTO = 0,    /* default: MGPCG for grids of 2^10 cells or more, CG below (faster there) */
+    FE_PRESSURE_MGPCG = 1,   /* CG preconditioned by one multigrid V-cycle: 7-15 inner iterations, about 2 L + 2 barriers each */
     FE_PRESSURE_CG = 2       /* unpreconditioned CG: one grid barrier per iteration, 130-1100 iterations */
 } fe_pressure_solver;
 
@@ -269,7 +269,8 @@ fe_status fe_volume_field_vectors(const double* vertices, uint64_t n_vertices, c
  * blocking, extrapolation and tangential projection at every ApplyBoundryCondition, and ResolveCollision in
  * MoveParticles with the reference's indexing (a particle ending inside the collider SDF moves particle number c
  * onto collider c's surface; pic_simulator.cpp:296-305).  At most 8; kept by fe_scene_reset.  A scene with
- * colliders uses the plain CG pressure solver, cannot join a batch and cannot have a viscosity > 0.
+ * colliders cannot join a batch and cannot have a viscosity > 0; substeps in which a collider shuts fluid in are solved by
+ * the plain CG.
  * fe_scene_get_collider_sdf returns the collider SDF as the reference holds it (0 before the first substep). */
 fe_status fe_scene_add_mesh_collider(fe_scene* s, const double* vertices, uint64_t n_vertices, const int64_t* triangles,
                                      uint64_t n_triangles, const double* normals, uint64_t n_normals,
