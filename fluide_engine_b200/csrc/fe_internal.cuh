@@ -72,7 +72,7 @@ struct SceneView {
     // the sort's scratch: key per particle; rank = a particle's atomic slot in its cell, then (after the sort) the
     // sorted order, slot -> particle; perm = the runs in arbitrary order; cell counts and starts per cell key
     uint32_t *key, *rank, *perm, *cell_count, *cell_start;
-    uint32_t* p2g_list;    // P2G: how many quarter tiles hold more than a few particles, then those
+    uint32_t* p2g_list;    // P2G: how many quarter tiles hold more than a few particles, how many are taken, then those
     // grid
     float *u, *v, *w;
     float *u2, *v2, *w2;

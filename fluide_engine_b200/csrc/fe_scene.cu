@@ -455,7 +455,7 @@ fe_status alloc_grid(fe_scene* s)
     FE_CUDA(dalloc(L, &v.cell_count, v.g.key_space, dev, st));
     FE_CUDA(dalloc(L, &v.cell_start, (size_t)v.g.key_space + 1, dev, st));
     FE_CUDA(cudaMemsetAsync(v.cell_start, 0, ((size_t)v.g.key_space + 1) * sizeof(uint32_t), st));
-    FE_CUDA(dalloc(L, &v.p2g_list, (size_t)p2g_blocks(v) + 1, dev, st));
+    FE_CUDA(dalloc(L, &v.p2g_list, (size_t)p2g_blocks(v) + 2, dev, st));
     s->scan_tmp_bytes = sort_scan_tmp_bytes(v.g.key_space);
     uint8_t* tmp;
     FE_CUDA(dalloc(L, &tmp, s->scan_tmp_bytes, dev, st));
