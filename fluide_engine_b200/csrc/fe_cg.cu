@@ -386,7 +386,10 @@ cudaError_t cg_prepare(CgWork& w, int device, int threads, int cluster)
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg, threads, 0);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(mgcg_kernel(threads), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mg_dynamic_smem(threads));
+    // the limit belongs to the kernel, not to this scene: the most that any of its block sizes needs, so that a scene of
+    // smaller blocks doesn't lower it for the others
+    e = cudaFuncSetAttribute(mgcg_kernel(threads), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)mg_dynamic_smem(threads < 512 ? threads : kCgThreads));
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_mg, mgcg_kernel(threads), threads, mg_dynamic_smem(threads));
     if (e != cudaSuccess) return e;

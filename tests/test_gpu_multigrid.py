@@ -55,3 +55,17 @@ def test_multigrid_solve_matches_oracle(n, h, kind):
     assert res <= 1e-12
     assert np.linalg.norm(p - expected) <= 1.03e-5 * np.linalg.norm(expected)
     g.close()
+
+
+def test_scenes_of_different_block_sizes():
+    """A scene of smaller solver blocks prepared after one of larger blocks, both stepped afterwards."""
+    scenes = []
+    for threads in (1024, 512, 256):
+        g = fe.Scene((32, 32, 32), solver=fe.FLIP, max_cfl=1.0)
+        g.set_tuning(multigrid=1, cg_block_threads=threads)
+        pos, _ = fe.seed_regions([dict(kind=0, lo=(0, 0, 0), hi=(0.4, 0.6, 1.0))], (32, 32, 32), (0, 0, 0), (1, 1, 1), 3)
+        g.set_particles(pos, np.zeros_like(pos))
+        scenes.append(g)
+    for g in scenes:
+        assert all(s["converged"] == 1 for s in g.step(1 / 240, 2))
+        g.close()
