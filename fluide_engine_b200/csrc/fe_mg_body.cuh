@@ -1361,8 +1361,17 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
                 alpha = (float)a;
             }
         }
-        // ---- p += e (FP64); the next residual pass reads neighbours' p, hence the barrier
-        for_cells([&](size_t c, uint32_t) { p64[c] = __ldcg(p64 + c) + (double)X[c]; });
+        // ---- p += e (FP64); the next residual pass reads neighbours' p, hence the barrier.  A tank full of fluid (no air, so
+        // no cell has a fixed pressure) determines p up to a constant: the plain CG keeps the mean that p starts with, while
+        // the preconditioner moves it, so the mean of e is taken out again (one more reduction per refinement, there only).
+        double mean = 0.0;
+        if ((size_t)F == nc) {
+            double xacc[1] = {0.0};
+            for_cells([&](size_t c, uint32_t) { xacc[0] += (double)X[c]; });
+            if (!grid_reduce<1>(xacc, sh, w, gen, nblk, blk)) return;
+            mean = xacc[0] / (double)F;
+        }
+        for_cells([&](size_t c, uint32_t) { p64[c] = __ldcg(p64 + c) + ((double)X[c] - mean); });
         if (!grid_sync(w, gen, nblk, sh, blk)) return;
     }
     if (blk == 0 && threadIdx.x == 0 && out_its) {
