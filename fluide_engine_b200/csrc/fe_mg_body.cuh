@@ -86,6 +86,7 @@ struct MgShared {
     uint32_t cache[kTileCache];        // the block's first tiles of each level
     uint32_t cache_at[kMaxMgLevels + 1];
     uint32_t scan[33];
+    double p_sum;                      // the sum of the starting pressure (a tank full of fluid)
 };
 
 template <int TEAM>
@@ -1189,6 +1190,20 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
 
     const double target = prm.rel_tol * bnorm;
     if (bnorm == 0.0) for_cells([&](size_t c, uint32_t) { p64[c] = 0.0; });
+    // A tank full of fluid (no air, so no cell has a fixed pressure) determines p up to a constant.  The plain CG keeps the mean
+    // that p starts with; the preconditioner moves it, so it is put back at the end.
+    auto p_sum = [&](double& sum) -> bool {
+        double pacc[1] = {0.0};
+        for (size_t c = (size_t)blk * blockDim.x + threadIdx.x; c < nc; c += (size_t)nblk * blockDim.x) pacc[0] += __ldcg(p64 + c);
+        const bool ok = grid_reduce<1>(pacc, sh, w, gen, nblk, blk);
+        sum = pacc[0];
+        return ok;
+    };
+    if ((size_t)F == nc) {
+        double sum;
+        if (!p_sum(sum)) return;
+        if (threadIdx.x == 0) ms.p_sum = sum;
+    }
     int total_it = 0, refinements = 0;
     double rnorm = 0.0, rho_old = 1.0;
     bool converged = bnorm == 0.0;
@@ -1361,18 +1376,15 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
                 alpha = (float)a;
             }
         }
-        // ---- p += e (FP64); the next residual pass reads neighbours' p, hence the barrier.  A tank full of fluid (no air, so
-        // no cell has a fixed pressure) determines p up to a constant: the plain CG keeps the mean that p starts with, while
-        // the preconditioner moves it, so the mean of e is taken out again (one more reduction per refinement, there only).
-        double mean = 0.0;
-        if ((size_t)F == nc) {
-            double xacc[1] = {0.0};
-            for_cells([&](size_t c, uint32_t) { xacc[0] += (double)X[c]; });
-            if (!grid_reduce<1>(xacc, sh, w, gen, nblk, blk)) return;
-            mean = xacc[0] / (double)F;
-        }
-        for_cells([&](size_t c, uint32_t) { p64[c] = __ldcg(p64 + c) + ((double)X[c] - mean); });
+        // ---- p += e (FP64); the next residual pass reads neighbours' p, hence the barrier
+        for_cells([&](size_t c, uint32_t) { p64[c] = __ldcg(p64 + c) + (double)X[c]; });
         if (!grid_sync(w, gen, nblk, sh, blk)) return;
+    }
+    if ((size_t)F == nc && refinements > 0) {
+        double sum;
+        if (!p_sum(sum)) return;
+        const double shift = (sum - ms.p_sum) / (double)F;
+        for (size_t c = (size_t)blk * blockDim.x + threadIdx.x; c < nc; c += (size_t)nblk * blockDim.x) p64[c] = __ldcg(p64 + c) - shift;
     }
     if (blk == 0 && threadIdx.x == 0 && out_its) {
         *out_its = total_it;
