@@ -452,12 +452,22 @@ int mg_plan(int nx, int ny, int nz, const double h[3], MgLevel* out)
     return levels;
 }
 
-int mg_block_from(const MgLevel* lv, int levels, int block_cells)
+int mg_block_from(const MgLevel* lv, int levels, int block_cells, int threads)
 {
-    int b = levels - 1;
-    while (b > 1 && (size_t)lv[b - 1].nx * lv[b - 1].ny * lv[b - 1].nz <= (size_t)block_cells) --b;
+    // the block's levels lie side by side in the memory of its tile teams (256 threads: 1612 cells in all, 512: 3224, 1024:
+    // 6452); the last one always fits
+    const size_t room = (size_t)(threads / 256) * sizeof(MgTeam);
+    size_t bytes = 0;
+    int b = levels;
+    while (b > 1) {
+        const size_t cells = (size_t)lv[b - 1].nx * lv[b - 1].ny * lv[b - 1].nz;
+        bytes += ((cells + 3) & ~(size_t)3) * kBlockCellBytes;
+        if (b < levels && (cells > (size_t)block_cells || bytes > room)) break;
+        --b;
+    }
     return b;
 }
+static_assert(kCoarseMaxCells * kBlockCellBytes <= sizeof(MgTeam), "the last level fits in the smallest block's memory");
 
 cudaError_t launch_mgcg(const SceneView& v, const CgWork& w, const MgWork& mg, double rel_tol, double inner_tol,
                         int max_it, int max_refine, cudaStream_t st, const uint32_t* gate)

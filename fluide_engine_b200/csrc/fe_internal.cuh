@@ -335,15 +335,15 @@ struct MgLevel {
 };
 struct MgWork {
     int levels;        // levels in use (0 or 1: no hierarchy, the plain CG solves)
-    int block_from;    // levels >= block_from (at most 4096 cells each) are processed by one block alone
+    int block_from;    // levels >= block_from are processed by one block alone (mg_block_from)
     MgLevel lv[kMaxMgLevels];
 };
 // Level dimensions for an nx x ny x nz grid with spacing h (host); returns the number of levels (>= 2), or 1
 // when the grid is too small for a hierarchy.
 int mg_plan(int nx, int ny, int nz, const double h[3], MgLevel* out);
-// First level (>= 1) from which every level has at most block_cells cells and is processed by one block without
-// grid barriers.
-int mg_block_from(const MgLevel* lv, int levels, int block_cells);
+// First level (>= 1) from which every level has at most block_cells cells and all fit in the shared memory of one block of
+// `threads` threads, which processes them without grid barriers.
+int mg_block_from(const MgLevel* lv, int levels, int block_cells, int threads);
 
 // One scene of a multi-scene pressure solve (fe_cg.cu k_multi_cg): the scene's grid view and solver
 // buffers, its solver settings and the block range [block_start, block_start + block_count) that solves it.

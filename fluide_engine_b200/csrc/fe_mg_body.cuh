@@ -580,9 +580,10 @@ __device__ __forceinline__ void coarse_up(MgTeam* teams, const MgShared& ms, con
     }
 }
 
-// ---- levels [LB, L), at most kBlockCellBytes of the block's memory per cell: the first block takes the whole lower part
-// of the V-cycle with the levels in shared memory, block barriers between the sweeps.  (One tile after the other through
-// global memory took 16 us for a 16^3 level and the 8^3 below it at 128^3, spread over the grid 13 us with its barriers.)
+// ---- levels [LB, L), at most kBlockCellBytes of the block's memory per cell (mg_block_from keeps to what it has): the first
+// block takes the whole lower part of the V-cycle with the levels in shared memory, block barriers between the sweeps.  (One
+// tile after the other through global memory took 16 us for a 16^3 level and the 8^3 below it at 128^3, spread over the grid
+// 13 us with its barriers.)
 constexpr int kBlockCellBytes = 17;
 struct BlockLevel {
     int nx, ny, nz, n;
@@ -782,18 +783,7 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
     uint8_t* flags = code + nc;  // one byte per tile, level after level
     uint32_t* list = w.list;     // listed tiles, level after level
     const int L = mg.levels;
-    int LB = mg.block_from;      // first level of the first block's share: what its memory holds
-    {
-        size_t bytes = 0;
-        int fit = L;
-        while (fit > 1) {
-            const MgLevel& M = mg.lv[fit - 1];
-            bytes += (size_t)((M.nx * M.ny * M.nz + 3) & ~3) * kBlockCellBytes;
-            if (bytes > (size_t)nteam * sizeof(MgTeam)) break;
-            --fit;
-        }
-        LB = max(LB, max(fit, 1));
-    }
+    const int LB = mg.block_from;  // first level of the first block's share (mg_block_from: its memory holds them)
     unsigned gen = 0;
     const bool solids = prm.gate != nullptr;  // a scene with colliders: there may be BOUNDRY cells
 

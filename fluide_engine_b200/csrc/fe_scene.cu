@@ -132,7 +132,7 @@ struct fe_scene {
     MgWork mg{};                       // multigrid levels (levels >= 2) once the multigrid solver was wanted
     bool use_mg = false;               // solve with the multigrid-preconditioned CG (if the grid has a hierarchy)
     double* pprev_buf = nullptr;       // pressure of the substep before the last (time-extrapolated warm start)
-    int mg_block_cells = 2048;         // multigrid levels of at most this many cells run in one block
+    int mg_block_cells = 2048;         // multigrid levels of at most this many cells run in one block if its memory holds them
     DiffWork diff{};                   // viscosity buffers (allocated once the viscosity is > 0)
     bool diff_ready = false;
     // Surface extraction (fe_surface.cu), allocated on first use: node distances and SDF values, per-item case
@@ -411,7 +411,7 @@ fe_status ensure_mg(fe_scene* s)
     }
     for (int l = 0; l < levels; ++l) s->mg.lv[l] = lv[l];
     s->mg.levels = levels;
-    s->mg.block_from = mg_block_from(s->mg.lv, levels, s->mg_block_cells);
+    s->mg.block_from = mg_block_from(s->mg.lv, levels, s->mg_block_cells, s->cg.threads);
     return FE_OK;
 }
 
@@ -471,6 +471,7 @@ fe_status alloc_grid(fe_scene* s)
     w.rws1 = reinterpret_cast<float4*>(vec + 4 * nc);
     w.xcg = vec + 8 * nc;
     FE_CUDA(dalloc(L, &w.list, nc, dev, st));
+    FE_CUDA(cg_prepare(w, s->device));
     // multigrid levels 1 .. L-1 (dense; level 0 is the grid above)
     s->mg.levels = 0;
     s->use_mg = s->desc.pressure_solver == FE_PRESSURE_MGPCG ||
@@ -479,7 +480,6 @@ fe_status alloc_grid(fe_scene* s)
         fe_status mst = ensure_mg(s);
         if (mst != FE_OK) return mst;
     }
-    FE_CUDA(cg_prepare(w, s->device));
     // 3 rotating totals slots (12 doubles) + per-block FLUID counts of up to kMaxCgBlocks solver blocks
     FE_CUDA(dalloc(L, &w.partial, cg_partial_doubles(kMaxCgBlocks), dev, st));
     FE_CUDA(cudaMemsetAsync(w.partial, 0, cg_partial_doubles(kMaxCgBlocks) * sizeof(double), st));
@@ -1183,10 +1183,8 @@ fe_status apply_tuning(fe_scene* s, const fe_tuning* t)
         s->cg.threads = w.threads;
         s->cg.cluster = w.cluster;
     }
-    if (t->mg_block_level_cells > 0) {
-        s->mg_block_cells = t->mg_block_level_cells;
-        if (s->mg.levels >= 2) s->mg.block_from = mg_block_from(s->mg.lv, s->mg.levels, s->mg_block_cells);
-    }
+    if (t->mg_block_level_cells > 0) s->mg_block_cells = t->mg_block_level_cells;
+    if (s->mg.levels >= 2) s->mg.block_from = mg_block_from(s->mg.lv, s->mg.levels, s->mg_block_cells, s->cg.threads);
     if (t->pressure_extrapolation > 1) return set_error(FE_ERR_BAD_ARG, "pressure_extrapolation is 0 or 1");
     if (t->pressure_extrapolation == 1 && !s->pprev_buf) {
         const size_t nc = (size_t)s->base.g.nx * s->base.g.ny * s->base.g.nz;
@@ -2524,6 +2522,10 @@ fe_status fe_scene_get_tuning(fe_scene* s, fe_tuning* t)
     t->multigrid = s->use_mg && s->mg.levels >= 2 ? 1 : 0;
     t->cg_block_threads = s->cg.threads;
     t->mg_block_level_cells = s->mg_block_cells;
+    if (t->multigrid && s->mg.block_from > 1) {  // a level of fewer cells that the block's memory doesn't hold bounds it
+        const MgLevel& M = s->mg.lv[s->mg.block_from - 1];
+        t->mg_block_level_cells = std::min(t->mg_block_level_cells, M.nx * M.ny * M.nz - 1);
+    }
     t->cg_cluster = std::max(s->cg.cluster, 1);
     t->pressure_extrapolation = s->base.pprev ? 1 : 0;
     return FE_OK;
@@ -2550,22 +2552,25 @@ fe_status fe_scene_autotune(fe_scene* s, double dt, int32_t substeps, int32_t sc
     if (!s || !(dt > 0.0) || substeps < 1 || scope < FE_TUNE_ALL || scope > FE_TUNE_SHAPE)
         return set_error(FE_ERR_BAD_ARG, "bad autotune arguments");
     if (!s->have_particles || s->base.np == 0) return set_error(FE_ERR_STATE, "autotune needs particles");
-    // candidates: the plain CG at 256 / 512 / 1024 threads per block and, where the grid has a multigrid hierarchy
-    // and no colliders, the multigrid-preconditioned CG at 512 / 1024 threads with one-block levels up to 2048 or
-    // 4096 cells
+    // candidates: the plain CG at 256 / 512 / 1024 threads per block and, where the grid has a multigrid hierarchy, the
+    // multigrid-preconditioned CG at 512 / 1024 threads with one-block levels up to 4096 or, where that makes a difference
+    // (mg_block_from), 2048 cells
     fe_tuning before;
     fe_status st = fe_scene_get_tuning(s, &before);
     if (st != FE_OK) return st;
     std::vector<fe_tuning> cand;
     MgLevel lv[kMaxMgLevels];
     const SceneView& b = s->base;
-    const bool mg_ok = mg_plan(b.g.nx, b.g.ny, b.g.nz, b.h, lv) >= 2;
+    const int levels = mg_plan(b.g.nx, b.g.ny, b.g.nz, b.h, lv);
+    const bool mg_ok = levels >= 2;
     if (scope == FE_TUNE_ALL || before.multigrid == 0)
         for (int th : {1024, 512, 256})
             for (int cl : {1, 2}) cand.push_back(fe_tuning{0, th, 4096, cl, -1});
     if (mg_ok && (scope == FE_TUNE_ALL || before.multigrid == 1))
         for (int th : {1024, 512})
-            for (int cells : {4096, 2048}) cand.push_back(fe_tuning{1, th, cells, 1, -1});
+            for (int cells : {4096, 2048})
+                if (cells == 4096 || mg_block_from(lv, levels, cells, th) != mg_block_from(lv, levels, 4096, th))
+                    cand.push_back(fe_tuning{1, th, cells, 1, -1});
     fe_snapshot* snap = nullptr;
     st = fe_scene_snapshot(s, &snap);
     if (st != FE_OK) return st;
@@ -3080,6 +3085,7 @@ fe_status batch_set_members(fe_batch* b, fe_scene* const* scenes, int32_t count)
         t.work = s->cg;
         t.work.cluster = 1;  // the multi-scene solve is not a cluster launch
         t.mg = s->mg;
+        if (t.mg.levels >= 2) t.mg.block_from = mg_block_from(t.mg.lv, t.mg.levels, s->mg_block_cells, threads);
         t.use_mg = s->use_mg && s->mg.levels >= 2 ? 1 : 0;
         t.rel_tol = s->desc.cg_rel_tol;
         t.inner_tol = inner_tol(s->desc, t.use_mg != 0);

@@ -320,7 +320,9 @@ fe_status fe_project_noalloc(const int32_t n[3], const double h[3], const uint8_
 typedef struct fe_tuning {
     int32_t multigrid;            /* 1: multigrid-preconditioned CG, 0: plain CG (grids too small for a hierarchy stay plain) */
     int32_t cg_block_threads;     /* threads per persistent solver block: 256, 512 or 1024 (1024 threads per SM in total) */
-    int32_t mg_block_level_cells; /* multigrid levels of at most this many cells are processed by one block */
+    int32_t mg_block_level_cells; /* multigrid levels of at most this many cells are processed by one block, as far as its
+                                     shared memory holds them (1612 cells in all per 256 threads); fe_scene_get_tuning
+                                     reports the limit in effect */
     int32_t cg_cluster;           /* thread-block cluster size of the persistent solve (1, 2, 4, 8, 16): the blocks of a
                                      cluster pre-reduce their sums in distributed shared memory and one block per
                                      cluster arrives at the grid barrier */
@@ -339,7 +341,8 @@ fe_status fe_scene_get_tuning(fe_scene* s, fe_tuning* t);
 enum { FE_TUNE_ALL = 0, FE_TUNE_SHAPE = 1 };
 /* The autotuner: times every candidate launch choice of the scene's pressure solve -- the plain CG at 256 / 512 /
  * 1024 threads per block, alone or in clusters of 2 blocks, and (grids with a multigrid hierarchy)
- * the multigrid-preconditioned CG at 512 / 1024 threads with one-block levels up to 2048 or 4096 cells; with
+ * the multigrid-preconditioned CG at 512 / 1024 threads with one-block levels up to 4096 or 2048 cells (where the two
+ * differ); with
  * FE_TUNE_SHAPE only the current family's --
  * over `substeps` substeps of dt each from the scene's current state (CUDA events on the scene's stream,
  * after one untimed substep that captures the choice's graphs), keeps the fastest whose solves all converged,
