@@ -797,10 +797,13 @@ MarkConst mark_constants(const SceneView& v)
     return mc;
 }
 
-// From this many particles on the two passes take less time than the one.  The marking stage with its clears and launches,
-// one pass against two: 0.5 M particles (64^3) 39 us against 43, 0.6 M (61x90x47) 51.5 against 52.5, 2 M (100^3) 73 against
-// 66, 4 M (128^3) 91 against 79; of the kernels alone 75 us against 50 at 128^3 and 1018 against 363 at 256^3 (32 M).
-constexpr uint64_t kMarkTwoPasses = 1ull << 19;
+// From this many particles on the two passes take less time than the one.  The passes before the solve, one marking pass
+// against two: 0.6 M particles (64^3) 105.5 us against 107, 0.8 M (72^3) 149 against 150.5, 1.1 M (80^3) 172 against 172,
+// 1.5 M (88^3) 206 against 203, 2 M (96^3) 252 against 239, 4.7 M (128^3) 520 against 490; of the kernels alone 75 against 50
+// at 128^3 and 1018 against 363 at 256^3 (32 M).  Grids with inexact cell-centre samples take them at half as many: there the
+// one pass lists the cell of every particle at a node's radius, also where another particle marks it, and fluid on a lattice
+// (80^3, 1 M) took 15.5 ms against 0.055.
+constexpr uint64_t kMarkTwoPasses = 1ull << 20, kMarkTwoPassesInexact = 1ull << 19;
 cudaError_t launch_mark(const SceneView& v, bool cells_current, cudaStream_t st)
 {
     const size_t nc = (size_t)v.g.nx * v.g.ny * v.g.nz;
@@ -813,7 +816,7 @@ cudaError_t launch_mark(const SceneView& v, bool cells_current, cudaStream_t st)
     }
     if (v.np > 0) {
         const unsigned nb = (unsigned)((v.np + 255) / 256);
-        if (mc.two && cells_current && v.np >= kMarkTwoPasses) {
+        if (mc.two && cells_current && v.np >= (v.any_inexact ? kMarkTwoPassesInexact : kMarkTwoPasses)) {
             k_mark_own<<<nb, 256, 0, st>>>(v, mc);
             k_mark_near<<<(unsigned)(v.g.tnx * v.g.tny * v.g.tnz), 256, 0, st>>>(v, mc);
             count_launch(2);
