@@ -1,6 +1,6 @@
-// fe_solver_common.cuh -- device pieces shared by the persistent pressure solvers (fe_cg.cu, fe_mgcg.cu):
-// the bounded grid barrier, grid-wide FP64 sums fused with it, the 7-point FLUID-row stencil and the setup
-// that compacts the FLUID cells into the solver's list.  Internal linkage: each solver file gets its own copy.
+// fe_solver_common.cuh -- device pieces of the persistent pressure solvers (fe_cg.cu, fe_mg_body.cuh) and the other
+// persistent kernels: the bounded grid barrier, grid-wide FP64 sums fused with it, the 7-point FLUID-row stencil and the
+// plain CG's setup, which compacts the FLUID cells into its list.  Internal linkage: each file gets its own copy.
 #pragma once
 
 #include <cuda/atomic>
@@ -340,23 +340,19 @@ __device__ __forceinline__ float apply_row(const Stencil7& st, int c, uint32_t m
     return st.ih2[0] * ax + st.ih2[1] * ay + st.ih2[2] * az;
 }
 
-// Shared memory of one solver block, declared once per kernel and handed to whichever solver body runs.
-constexpr int kCoarseMaxCells = 512;  // the multigrid solver's coarsest level lives in shared memory
+constexpr int kCoarseMaxCells = 512;  // the multigrid solver's coarsest level lives in one block's shared memory
+// Shared memory of one block of the plain CG.
 struct SolverSmem {
     double sh[kShDoubles];                 // block reductions, then the cluster pre-reduction's words
     uint32_t s_warp[32];                   // compaction counts
     uint32_t s_list[kListCache];           // cached FLUID-list entries
 };
 
-// Solver setup shared by the persistent solvers, run by `nblk` blocks of which this is block `blk`: zeroes
-// the non-FLUID entries of the pressure and of the FP32 solver vectors (so stencils over them need no branch
-// on the cell type), sums ||b||^2, compacts the FLUID cells in cell order into w.list with their
-// in-domain-neighbour masks (per-block counts -> grid reduction -> block offsets -> ordered compaction), and
-// caches each thread's first list entries in s_list.  Returns false when a grid wait gave up.
-// Vector layouts whose non-FLUID entries the setup zeroes: the multigrid solver's separate arrays, the plain CG's
-// interleaved (r, w, s, p) cells.
-enum { kLayoutSeparate = 0, kLayoutInterleaved = 1 };
-
+// The plain CG's setup, run by `nblk` blocks of which this is block `blk`: zeroes the non-FLUID entries of the pressure
+// and of its interleaved (r, w, s, p) cells (so stencils over them need no branch on the cell type), sums ||b||^2,
+// compacts the FLUID cells in cell order into w.list with their in-domain-neighbour masks (per-block counts -> grid
+// reduction -> block offsets -> ordered compaction), and caches each thread's first list entries in s_list.  Returns
+// false when a grid wait gave up.
 struct SolverSetup {
     int F;          // FLUID cells
     double bnorm;   // ||b||_2
@@ -387,7 +383,7 @@ __device__ __forceinline__ uint32_t solve_mask(const uint8_t* __restrict__ marks
 
 __device__ __forceinline__ bool solver_setup(const SceneView& v, const CgWork& w, const int blk, const int nblk,
                                              unsigned& gen, double* sh, uint32_t* s_warp, uint32_t* s_list,
-                                             SolverSetup& out, int layout)
+                                             SolverSetup& out)
 {
     const int nx = v.g.nx, ny = v.g.ny, nz = v.g.nz;
     const int sxy = nx * ny;
@@ -397,9 +393,6 @@ __device__ __forceinline__ bool solver_setup(const SceneView& v, const CgWork& w
     const uint8_t* __restrict__ marks = v.marks;
     double* __restrict__ p64 = v.p;
     const double* __restrict__ b = v.b;
-    float* __restrict__ R[2] = {w.r0, w.r1};
-    float* __restrict__ W[2] = {w.w0, w.w1};
-    float* __restrict__ S[2] = {w.s0, w.s1};
     uint32_t* __restrict__ list = w.list;
     gen = 0;  // barriers passed in this launch
 
@@ -413,18 +406,8 @@ __device__ __forceinline__ bool solver_setup(const SceneView& v, const CgWork& w
             acc[1] += 1.0;
         } else {
             p64[c] = 0.0;
-            if (layout == kLayoutInterleaved) {  // the single-pass CG's (r, w, s, p) cells
-                w.rws0[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-                w.rws1[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-            } else {
-                R[0][c] = 0.f;
-                R[1][c] = 0.f;
-                W[0][c] = 0.f;
-                W[1][c] = 0.f;
-                S[0][c] = 0.f;
-                S[1][c] = 0.f;
-                w.pv[c] = 0.f;
-            }
+            w.rws0[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+            w.rws1[c] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
     // block offset = FLUID count of all earlier blocks (fixed order), total = all blocks
