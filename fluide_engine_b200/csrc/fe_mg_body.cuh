@@ -93,7 +93,7 @@ struct MgShared {
     uint32_t cache[kTileCache];        // the block's first tiles of each level
     uint32_t cache_at[kMaxMgLevels + 1];
     uint32_t scan[33];
-    double p_sum;                      // the sum of the starting pressure (a tank full of fluid)
+    double p_sum[2];                   // a tank full of fluid: the sum of the starting pressure and the present one's
 };
 
 template <int TEAM>
@@ -1191,20 +1191,6 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
 
     const double target = prm.rel_tol * bnorm;
     if (bnorm == 0.0) for_cells([&](size_t c, uint32_t) { p64[c] = 0.0; });
-    // A tank full of fluid (no air, so no cell has a fixed pressure) determines p up to a constant.  The plain CG keeps the mean
-    // that p starts with; the preconditioner moves it, so it is put back at the end.
-    auto p_sum = [&](double& sum) -> bool {
-        double pacc[1] = {0.0};
-        for (size_t c = (size_t)blk * blockDim.x + threadIdx.x; c < nc; c += (size_t)nblk * blockDim.x) pacc[0] += __ldcg(p64 + c);
-        const bool ok = grid_reduce<1>(pacc, sh, w, gen, nblk, blk);
-        sum = pacc[0];
-        return ok;
-    };
-    if ((size_t)F == nc) {
-        double sum;
-        if (!p_sum(sum)) return;
-        if (threadIdx.x == 0) ms.p_sum = sum;
-    }
     int total_it = 0, refinements = 0;
     double rnorm = 0.0, rho_old = 1.0;
     bool converged = bnorm == 0.0;
@@ -1233,6 +1219,12 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
             for (int c = (int)threadIdx.x; c < mg.lv[1].nx * mg.lv[1].ny * mg.lv[1].nz; c += (int)blockDim.x) mg.lv[1].r[c] = 0.f;
         if (!grid_reduce<1>(racc, sh, w, gen, nblk, blk)) return;
         rnorm = sqrt(racc[0]);
+        if ((size_t)F == nc) {  // the sum of p, at first and now
+            racc[0] = 0.0;
+            for_cells([&](size_t c, uint32_t) { racc[0] += __ldcg(p64 + c); });
+            if (!grid_reduce<1>(racc, sh, w, gen, nblk, blk)) return;
+            if (threadIdx.x == 0) ms.p_sum[refinements > 0] = racc[0];
+        }
         if (rnorm <= target) {
             converged = true;
             break;
@@ -1381,10 +1373,11 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
         for_cells([&](size_t c, uint32_t) { p64[c] = __ldcg(p64 + c) + (double)X[c]; });
         if (!grid_sync(w, gen, nblk, sh, blk)) return;
     }
+    // A tank full of fluid (no air, so no cell has a fixed pressure) determines p up to a constant.  The plain CG keeps the mean
+    // that p starts with; the preconditioner moves it, so it is put back.
     if ((size_t)F == nc && refinements > 0) {
-        double sum;
-        if (!p_sum(sum)) return;
-        const double shift = (sum - ms.p_sum) / (double)F;
+        __syncthreads();
+        const double shift = (ms.p_sum[1] - ms.p_sum[0]) / (double)F;
         for (size_t c = (size_t)blk * blockDim.x + threadIdx.x; c < nc; c += (size_t)nblk * blockDim.x) p64[c] = __ldcg(p64 + c) - shift;
     }
     if (blk == 0 && threadIdx.x == 0 && out_its) {
