@@ -15,7 +15,7 @@ fe = pytest.importorskip("fluide_engine_b200")
 DT = 1 / 240
 EXACT = ((40, 56, 48), 1 / 64, (0, 0, 0))
 GRIDS = [EXACT, ((47, 41, 58), 1 / 60, (0, 0, 0)), ((50, 48, 44), 1 / 50, (-0.5, 0.25, 1.0))]
-KINDS = ["block", "spray", "corners", "crowded", "lattice"]
+KINDS = ["block", "spray", "corners", "crowded", "cap", "lattice"]
 
 
 def particles(n, h, origin, kind, count, rng):
@@ -29,6 +29,11 @@ def particles(n, h, origin, kind, count, rng):
         at = (rng.integers(0, n, (count // 60, 3)) + 0.5) * h
         pos = np.repeat(at, rng.integers(20, 140, len(at)), axis=0)
         pos = pos + rng.uniform(-0.6, 0.6, pos.shape) * h
+    elif kind == "cap":  # one cell each, around the 64 particles that 8 lanes test, and some hundreds and thousands
+        cells = rng.permutation(np.argwhere(np.ones(n, bool)))[:count // 62]
+        reps = rng.choice([61, 62, 63, 64, 65, 66, 67], len(cells))
+        reps[:7] = [255, 256, 257, 1023, 1025, 2049, 3000]
+        pos = (np.repeat(cells, reps, axis=0) + rng.uniform(0, 1, (reps.sum(), 3))) * h
     else:  # a block of fluid, 3^3 a cell; on a lattice of 5 x 5 x 1 some are 0.6 h away from a node along x and y: its radius
         per = np.array([3, 3, 3] if kind != "lattice" else [5, 5, 1])
         m = np.stack(np.meshgrid(*[np.arange(p * k) for p, k in zip(per, n)], indexing="ij"), -1).reshape(-1, 3)
