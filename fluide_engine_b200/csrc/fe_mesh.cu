@@ -19,8 +19,9 @@
 // signs of a closed mesh come from the grid rows: away from the surface its winding sum is 2 pi times an integer that
 // changes only where a row crosses a triangle, so one pass over the triangles records the crossings and one over the
 // rows adds them up; nodes whose row passes within rounding of an edge, or whose crossing lies within 1e-6 cells of a
-// node, sum the winding terms of all triangles, a warp per node.  Of an open mesh every node does, one thread per node
-// (fe_mesh_to_sdf of 1280 triangles on 96^3 nodes, copies included: 13.2 ms that way, 1.6 ms by rows).  The distance arithmetic follows the
+// node, sum the winding terms of all triangles, in a pass of their own.  Of an open mesh every node does, one thread per node
+// (fe_mesh_to_sdf of 1280 triangles on 96^3 nodes, copies included: 13.2 ms that way, 1.3 ms by rows).  The distance
+// arithmetic follows the
 // reference's expressions in FP64 with round-to-nearest intrinsics, so distances are bit-identical; the sign test
 // sums CUDA's atan2, whose last bits can differ from the host library's, which decides nothing unless a node lies
 // within ~1e-12 of the 2 pi - 0.001 threshold (points on the surface sum to pi, points inside to 2 pi).  Seeding
@@ -67,7 +68,7 @@ __global__ void __launch_bounds__(256) k_mesh_band(MeshView m, NodeGrid g, unsig
 // other.  Each use adds a hash of the undirected edge, with its direction as the sign, to two 64-bit sums, which are
 // zero for a closed mesh (and for an open one with probability 2^-128).  Then the solid angles of its triangles sum to
 // an integer times 4 pi at every point off the surface.  state: the two sums, then non-zero if a coordinate is not
-// finite.
+// finite.  mix64 is the output function of the splitmix64 generator (Steele, Lea and Flood 2014).
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z)
 {
     z += 0x9E3779B97F4A7C15ull;
@@ -128,12 +129,14 @@ __device__ __forceinline__ bool mesh_closed(const unsigned long long* state)
 
 // Crossings of the grid rows along x with the triangles of a closed mesh, a warp per triangle, a lane per row.  cross[c]:
 // .x the change of the winding number (half the winding sum over pi) from node c - 1 to c of the row -- at the first
-// node, from far to the left --, .y non-zero where the node is to sum the winding terms itself.  Going in +x through a
+// node, from far to the left --, bit 0 of .y set where the node is to sum the winding terms itself.  Those nodes are listed: the
+// k-th one in the other bits of cross[k].y (on grids that 31 bits can index), state[3] of them.  Going in +x through a
 // triangle whose projection on (y, z) is positively oriented leaves the side its normal points away from: -1.
 // The projected point is in the triangle when its three edge functions have one sign; `tol` bounds their rounding.
-__global__ void __launch_bounds__(256) k_mesh_cross(MeshView m, NodeGrid g, const unsigned long long* __restrict__ state,
-                                                    int2* __restrict__ cross)
+__host__ __device__ __forceinline__ bool mesh_listed(const NodeGrid& g) { return (size_t)g.n[0] * g.n[1] * g.n[2] < (1ull << 31); }
+__global__ void __launch_bounds__(256) k_mesh_cross(MeshView m, NodeGrid g, unsigned long long* state, int2* cross)
 {
+    const bool listed = mesh_listed(g);
     if (!mesh_closed(state)) return;
     const int lane = threadIdx.x & 31;
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
@@ -188,8 +191,61 @@ __global__ void __launch_bounds__(256) k_mesh_cross(MeshView m, NodeGrid g, cons
             if (from <= to) {
                 from = max(from, 0);
                 to = min(max(to, 0), g.n[0] - 1);  // left of the grid: the row's first node
-                for (int i = from; i <= to; ++i) cross[idx3(i, j, k, g.n[0], g.n[1])].y = 1;
+                for (int i = from; i <= to; ++i) {
+                    const size_t c = idx3(i, j, k, g.n[0], g.n[1]);
+                    if ((atomicOr(&cross[c].y, 1) & 1) || !listed) continue;
+                    atomicOr(&cross[atomicAdd(state + 3, 1ull)].y, (int)((unsigned)c << 1));
+                }
             }
+        }
+    }
+}
+
+// The side of a point by its winding sum: inside or not, its winding number, and whether that holds beside the point too (it
+// does not on the surface).
+struct Winding {
+    int w;
+    bool in, known;
+};
+__device__ __forceinline__ Winding winding(double sum)
+{
+    const double pi = 3.14159265358979323846;
+    const double turns = sum / (2.0 * pi);
+    Winding r;
+    r.in = fabs(sum) >= ds(dm(2.0, pi), 0.001);
+    r.w = (int)rint(turns);
+    r.known = fabs(turns - rint(turns)) < 1e-4;
+    return r;
+}
+
+// The listed nodes' winding sums: w << 2 | known << 1 | inside in cross[c].x, which holds no crossing that matters there.  2^k
+// lanes a node: all 32 for a few nodes, one where the nodes alone fill the device (then a warp's lanes read the same triangle).
+// A box of 12,288 triangles with its faces on the nodes of a 96^3 grid: 14.4 ms, 38.7 with every row's nodes summed one after the
+// other by the row's warp, 119 with no rows and a thread per node of the grid; with all 2 x 2 x 1024 nodes of a grid on its
+// surface 1.3, 308 and 10.7 ms.
+constexpr uint64_t kWindingLanes = 148 * 1024;
+__global__ void __launch_bounds__(256) k_mesh_own(MeshView m, NodeGrid g, const unsigned long long* __restrict__ state, int2* cross)
+{
+    if (!mesh_closed(state)) return;
+    const uint64_t n = mesh_listed(g) ? state[3] : 0;
+    int lanes = 32;
+    while (lanes > 1 && n * (uint64_t)lanes > kWindingLanes) lanes >>= 1;
+    const int lane = threadIdx.x & 31, sub = lane & (lanes - 1), per = 32 / lanes;
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    for (uint64_t e0 = (blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5)) * per; e0 < n; e0 += warps * per) {
+        const uint64_t e = e0 + lane / lanes;
+        const unsigned c = e < n ? (unsigned)cross[e].y >> 1 : 0u;
+        double sum = 0.0;
+        if (e < n) {
+            const unsigned row = c / (unsigned)g.n[0];
+            const double pt[3] = {grid_pos(g, 0, (int)(c % (unsigned)g.n[0])), grid_pos(g, 1, (int)(row % (unsigned)g.n[1])),
+                                  grid_pos(g, 2, (int)(row / (unsigned)g.n[1]))};
+            sum = winding_sum(m, pt, (uint64_t)sub, (uint64_t)lanes);
+        }
+        for (int o = lanes >> 1; o > 0; o >>= 1) sum = da(sum, __shfl_xor_sync(0xffffffffu, sum, o));
+        if (e < n && sub == 0) {
+            const Winding r = winding(sum);
+            cross[c].x = r.w * 4 + (r.known ? 2 : 0) + (r.in ? 1 : 0);
         }
     }
 }
@@ -197,13 +253,13 @@ __global__ void __launch_bounds__(256) k_mesh_cross(MeshView m, NodeGrid g, cons
 // TriangleMesh::IsInside at every node, then the signed value: -d inside, d outside.  k_mesh_rows: a closed mesh, a
 // warp per row, from the crossings (which share memory with the result: each lane reads its node's before it writes
 // it).  A node that sums for itself fixes the winding number for the nodes after it, unless it lies on the surface;
-// then the next one sums too.  k_mesh_sign: an open mesh, a thread per node.
+// then the next one sums too, which the row's warp does where k_mesh_own has not.  k_mesh_sign: an open mesh, a thread per
+// node.
 __global__ void __launch_bounds__(256) k_mesh_rows(MeshView m, NodeGrid g, const unsigned long long* __restrict__ state,
                                                    const unsigned long long* __restrict__ bits, double* sdf)
 {
     if (!mesh_closed(state)) return;
-    const double pi = 3.14159265358979323846;
-    const double two_pi_tol = ds(dm(2.0, pi), 0.001);
+    const bool listed = mesh_listed(g);
     const int2* cross = reinterpret_cast<const int2*>(sdf);
     const int lane = threadIdx.x & 31;
     const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5), rows = (size_t)g.n[1] * g.n[2];
@@ -215,7 +271,7 @@ __global__ void __launch_bounds__(256) k_mesh_rows(MeshView m, NodeGrid g, const
             const int i = i0 + lane, count = min(32, g.n[0] - i0);
             const size_t c = idx3(i, j, k, g.n[0], g.n[1]);
             const int2 x = lane < count ? cross[c] : make_int2(0, 0);
-            const unsigned own = __ballot_sync(0xffffffffu, x.y != 0);
+            const unsigned own = __ballot_sync(0xffffffffu, x.y & 1);
             bool inside = false;
             if (known && own == 0u) {
                 int s = x.x;
@@ -230,15 +286,19 @@ __global__ void __launch_bounds__(256) k_mesh_rows(MeshView m, NodeGrid g, const
                 for (int q = 0; q < count; ++q) {
                     const int step = __shfl_sync(0xffffffffu, x.x, q);
                     bool in;
-                    if (!known || ((own >> q) & 1u)) {
+                    if (listed && ((own >> q) & 1u)) {
+                        w = step >> 2;
+                        known = step & 2;
+                        in = step & 1;
+                    } else if (!known || ((own >> q) & 1u)) {
                         const double pt[3] = {grid_pos(g, 0, i0 + q), grid_pos(g, 1, j), grid_pos(g, 2, k)};
                         double sum = winding_sum(m, pt, (uint64_t)lane, 32);
 #pragma unroll
                         for (int o = 16; o > 0; o >>= 1) sum = da(sum, __shfl_xor_sync(0xffffffffu, sum, o));
-                        in = fabs(sum) >= two_pi_tol;
-                        const double turns = sum / (2.0 * pi);
-                        w = (int)rint(turns);
-                        known = fabs(turns - rint(turns)) < 1e-4;
+                        const Winding r = winding(sum);
+                        w = r.w;
+                        known = r.known;
+                        in = r.in;
                     } else {
                         w += step;
                         in = w != 0;
@@ -405,9 +465,10 @@ cudaError_t launch_mesh_to_sdf(const double* V, uint64_t nv, const int64_t* T, u
         k_mesh_closed<<<(unsigned)std::min<uint64_t>((nt + 255) / 256, 148 * 8), 256, 0, st>>>(m, state);
         k_mesh_cross<<<(unsigned)std::min<uint64_t>((nt + 7) / 8, 148 * 8), 256, 0, st>>>(m, g, state,
                                                                                          reinterpret_cast<int2*>(sdf));
+        k_mesh_own<<<148 * 8, 256, 0, st>>>(m, g, state, reinterpret_cast<int2*>(sdf));
         k_mesh_rows<<<(unsigned)std::min<size_t>(((size_t)n[1] * n[2] + 7) / 8, 148 * 32), 256, 0, st>>>(m, g, state, scratch,
                                                                                                        sdf);
-        count_launch(3);
+        count_launch(4);
     }
     k_mesh_sign<<<(unsigned)std::min<size_t>((nc + 255) / 256, 148 * 32), 256, 0, st>>>(m, g, state, scratch, sdf);
     count_launch();
