@@ -533,7 +533,8 @@ struct NodeShared {
     uint16_t row[kNodeHalo * kNodeHaloZ];  // occupied cells of a row, a bit each
     uint8_t near[FE_TILE * kNodeLayers];   // nodes of a row with an occupied cell that reaches into their band
     uint16_t list[kNodeThreads];           // nodes to search, a thread each
-    uint16_t hard[kNodeThreads];           // ... a warp each
+    uint16_t hard[kNodeThreads];           // ... the crowded cells, a warp each
+    double best[kNodeThreads];             // of those: the smallest squared distance in the other cells
     double near2[kNodeCells];
     int16_t cell[kNodeCells];              // offset in start and count
     int n, nhard;
@@ -693,8 +694,11 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
                 else full = true;
             }
         }
-        if (full) sh.hard[atomicAdd(&sh.nhard, 1)] = (uint16_t)t;
-        else out[idx3(i, j, k, nx, ny)] = value(best);
+        if (full) {
+            const int e = atomicAdd(&sh.nhard, 1);
+            sh.hard[e] = (uint16_t)t;
+            sh.best[e] = best;
+        } else out[idx3(i, j, k, nx, ny)] = value(best);
     }
     __syncthreads();
 
@@ -711,8 +715,8 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
         const int lx = t & 7, ly = (t >> 3) & 7, lz = t >> 6;
         const int i = x0 + lx, j = y0 + ly, k = z0 + lz;
         const double qx = v.q_pos[0][i], qy = v.q_pos[1][j], qz = v.q_pos[2][k];
-        double best = beyond;
-        for (int first = 0; first < kNodeCells; first += 32) {  // each lane its cell
+        double best = sh.best[e];
+        for (int first = 0; first < kNodeCells; first += 32) {  // each lane looks at a cell
             const int c = first + lane;
             uint32_t s = 0, n = 0;
             if (c < kNodeCells && sh.near2[c] < best) {
@@ -720,17 +724,16 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
                 s = sh.start[q];
                 n = sh.count[q];
             }
-            if (n <= kNodeLaneCap)
-                for (uint32_t m = 0; m < n; ++m) test(s + m, i, j, k, qx, qy, qz, best);
             unsigned full = __ballot_sync(0xffffffffu, n > kNodeLaneCap);
             while (full) {
                 const int from = __ffs(full) - 1;
                 full &= full - 1;
+                if (!(sh.near2[first + from] < best)) continue;
                 const uint32_t fs = __shfl_sync(0xffffffffu, s, from), fn = __shfl_sync(0xffffffffu, n, from);
                 for (uint32_t m = (uint32_t)lane; m < fn; m += 32) test(fs + m, i, j, k, qx, qy, qz, best);
-            }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) best = fmin(best, __shfl_xor_sync(0xffffffffu, best, o));
+                for (int o = 16; o > 0; o >>= 1) best = fmin(best, __shfl_xor_sync(0xffffffffu, best, o));
+            }
         }
         if (lane == 0) out[idx3(i, j, k, nx, ny)] = value(best);
     }
@@ -892,10 +895,18 @@ static bool node_reach(const SceneView& v, NodeReach& r)
     return ok;
 }
 
+// From this many particles on the gather from cells is taken rather than the scatter by particles: where the cells are known, and
+// where the particles have to be grouped first.  The gather's searches grow with the surface and wait for one another where few
+// tiles hold fluid, the scatter's work is the particles'.  us before the solve of scenes with a collider, scatter / gather, 3 and
+// 300 substeps into a dam break: 0.06 M particles (32^3) 161 / 170 and 200 / 278, 0.2 M (48^3) 193 / 202 and 240 / 305, 0.34 M
+// (56^3) 221 / 193 and 288 / 307, 0.5 M (64^3) 287 / 257 and 344 / 352, 1 M (80^3) 427 / 345 and 525 / 563.  Surfaces, the
+// gather with its grouping: 0.06 M 153 / 198 and 171 / 223, 0.5 M 204 / 210 and 229 / 240, 0.7 M (72^3) 218 / 191 and 246 / 287,
+// 1 M (80^3) 256 / 206 and 281 / 362, 1.7 M (96^3) 362 / 248 and 444 / 516, 4 M (128^3) 669 / 399 and 843 / 847.
+constexpr uint64_t kGatherKnown = 1ull << 18, kGatherGrouped = 1ull << 20;
 bool node_sdf_uses_cells(const SceneView& v)
 {
     NodeReach r;
-    return v.np > 0 && node_reach(v, r);
+    return v.np >= kGatherGrouped && node_reach(v, r);
 }
 
 cudaError_t launch_node_sdf(const SceneView& v, const NodeCells& cells, double* sdf, cudaStream_t st)
@@ -903,7 +914,7 @@ cudaError_t launch_node_sdf(const SceneView& v, const NodeCells& cells, double* 
     const size_t nc = (size_t)v.g.nx * v.g.ny * v.g.nz;
     const double R2 = v.band * v.band;
     NodeReach r;
-    if (v.np > 0 && cells.start && node_reach(v, r)) {
+    if (v.np >= kGatherKnown && cells.start && node_reach(v, r)) {
         const unsigned blocks = 2u * (unsigned)(v.g.tnx * v.g.tny * v.g.tnz);
         if (cells.order) k_sdf_gather<true><<<blocks, kNodeThreads, 0, st>>>(v, cells.start, cells.order, r, R2, sdf);
         else k_sdf_gather<false><<<blocks, kNodeThreads, 0, st>>>(v, cells.start, nullptr, r, R2, sdf);
