@@ -371,7 +371,7 @@ cudaError_t launch_mgcg(const SceneView& v, const CgWork& w, const MgWork& mg, d
 // each); counts per item, then the mesh from the scanned counts.
 size_t mc_items(int nx, int ny, int nz);
 cudaError_t launch_mc_count(const SceneView& v, const double* sdf, uint8_t* cfg, uint32_t* nvert, uint32_t* ntri,
-                            uint32_t* active /* count, then the items with triangles */, cudaStream_t st);
+                            uint32_t* active /* the items with triangles */, uint32_t* n_active, cudaStream_t st);
 cudaError_t launch_mc_emit(const SceneView& v, const double* sdf, const uint32_t* active, uint32_t n_active, const uint8_t* cfg,
                            const uint32_t* vbase, const uint32_t* tbase, double* V, double* N, int64_t* T, cudaStream_t st);
 

@@ -142,7 +142,7 @@ struct fe_scene {
         double* sdf = nullptr;
         uint8_t* cfg = nullptr;
         uint32_t *nvert = nullptr, *ntri = nullptr, *vbase = nullptr, *tbase = nullptr;
-        uint32_t* active = nullptr;                             // the items with triangles
+        uint32_t* active = nullptr;                             // the items with triangles, how many last
         uint32_t *cell_count = nullptr, *cell_start = nullptr;  // the particles by cell, for the SDF
         void* tmp = nullptr;
         size_t tmp_bytes = 0, items = 0;
@@ -1050,9 +1050,10 @@ fe_status surf_alloc(fe_scene* s)
         FE_CUDA(dalloc(L, &w.cfg, w.items, s->device, st));
         FE_CUDA(dalloc(L, &w.nvert, w.items, s->device, st));
         FE_CUDA(dalloc(L, &w.ntri, w.items, s->device, st));
-        FE_CUDA(dalloc(L, &w.vbase, w.items + 1, s->device, st));
-        FE_CUDA(dalloc(L, &w.tbase, w.items + 1, s->device, st));
-        FE_CUDA(dalloc(L, &w.active, w.items + 1, s->device, st));
+        // three rows whose last words are the mesh's sizes, so that one copy fetches them
+        FE_CUDA(dalloc(L, &w.vbase, 3 * (w.items + 1), s->device, st));
+        w.tbase = w.vbase + (w.items + 1);
+        w.active = w.tbase + (w.items + 1);
         FE_CUDA(dalloc(L, &w.cell_count, b.g.key_space, s->device, st));
         FE_CUDA(dalloc(L, &w.cell_start, (size_t)b.g.key_space + 1, s->device, st));
         uint8_t* tmp;
@@ -2207,13 +2208,12 @@ fe_status fe_scene_build_surface(fe_scene* s, uint64_t* n_vertices, uint64_t* n_
         FE_CUDA(launch_surface_with_colliders(w.sdf, s->cw.csdf, (size_t)v.g.nx * v.g.ny * v.g.nz, mod, stream));
         msdf = mod;
     }
-    FE_CUDA(launch_mc_count(v, msdf, w.cfg, w.nvert, w.ntri, w.active, stream));
+    FE_CUDA(launch_mc_count(v, msdf, w.cfg, w.nvert, w.ntri, w.active, w.active + w.items, stream));
     FE_CUDA(launch_exclusive_scan(w.nvert, (uint32_t)w.items, w.vbase, w.tmp, w.tmp_bytes, stream));
     FE_CUDA(launch_exclusive_scan(w.ntri, (uint32_t)w.items, w.tbase, w.tmp, w.tmp_bytes, stream));
     uint32_t tot[3] = {0, 0, 0};
-    FE_CUDA(cudaMemcpyAsync(&tot[2], w.active, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-    FE_CUDA(cudaMemcpyAsync(&tot[0], w.vbase + w.items, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-    FE_CUDA(cudaMemcpyAsync(&tot[1], w.tbase + w.items, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+    FE_CUDA(cudaMemcpy2DAsync(tot, sizeof(uint32_t), w.vbase + w.items, (w.items + 1) * sizeof(uint32_t), sizeof(uint32_t), 3,
+                              cudaMemcpyDeviceToHost, stream));
     FE_CUDA(cudaStreamSynchronize(stream));
     if (tot[0] > w.cap_v || tot[1] > w.cap_t) {
         free_list(w.mesh_allocs, stream);

@@ -12,8 +12,7 @@
 // use every crossed edge (and every inside corner of a square), so all items around a key create or look it up,
 // and the one that creates it is the first of them in sweep order -- a closed-form function of the key (along
 // each axis across the key, the item with the smaller index when both exist).  So:
-//   k_mc_count_cubes, k_mc_count_caps  per item: the case byte, its triangles and the keys it creates, and a list of
-//               the items with triangles;
+//   k_mc_count  per item: the case byte, its triangles and the keys it creates, and a list of the items with triangles;
 //   two exclusive scans over items give each item its first vertex and first triangle;
 //   k_mc_emit   per listed item: creates its keys' vertices (position, normal) at base + rank in its
 //               own use order, and resolves the other keys to the creating item's base + rank, recomputed from
@@ -182,7 +181,8 @@ __device__ int creation_rank(int kind, int side, const int c[3], int cfg, int ta
 // each its place).  All lanes of the warp take part; `on`: the lane has an item.
 __device__ __forceinline__ void count_item(const McGrid& g, bool on, uint64_t t, const Item& it, int cfg,
                                            uint8_t* __restrict__ cfg_out, uint32_t* __restrict__ nvert,
-                                           uint32_t* __restrict__ ntri, uint32_t* __restrict__ active)
+                                           uint32_t* __restrict__ ntri, uint32_t* __restrict__ active,
+                                           uint32_t* __restrict__ n_active)
 {
     int created = 0, nt = 0;
     if (on && cfg != 0 && !(it.kind == 0 && cfg == 255)) {
@@ -207,27 +207,46 @@ __device__ __forceinline__ void count_item(const McGrid& g, bool on, uint64_t t,
     if (some) {
         const int lane = (int)threadIdx.x & 31;
         uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(active, (uint32_t)__popc(some));
+        if (lane == 0) base = atomicAdd(n_active, (uint32_t)__popc(some));
         base = __shfl_sync(0xffffffffu, base, 0);
-        if (nt > 0) active[1 + base + __popc(some & ((1u << lane) - 1u))] = (uint32_t)t;
+        if (nt > 0) active[base + __popc(some & ((1u << lane) - 1u))] = (uint32_t)t;
     }
 }
 
-// The cubes of 32 x 1 x 32 cells a block.  The items run along z and the SDF along x, so a block turns the signs of its
-// nodes in shared memory: both sides then move in whole lines (with a thread per item reading its 8 nodes 75 us at 128^3).
+// The first blocks take the cubes of 32 x 1 x W cells each, the others the cap squares, an item a thread.  The items run along z
+// and the SDF along x, so a block turns the signs of its nodes in shared memory: both sides then move in whole lines (with a
+// thread per item reading its 8 nodes 75 us at 128^3).  W = 32 on large grids; 8 where that leaves SMs without a block.
 constexpr int kMcW = 32;
-__global__ void __launch_bounds__(256) k_mc_count_cubes(McGrid g, uint8_t* __restrict__ cfg_out, uint32_t* __restrict__ nvert,
-                                                        uint32_t* __restrict__ ntri, uint32_t* __restrict__ active)
+struct McCubeBlocks {
+    unsigned x, y, z;
+};
+template <int W>
+__global__ void __launch_bounds__(256) k_mc_count(McGrid g, McCubeBlocks nb, uint64_t items, uint8_t* __restrict__ cfg_out,
+                                                  uint32_t* __restrict__ nvert, uint32_t* __restrict__ ntri,
+                                                  uint32_t* __restrict__ active, uint32_t* __restrict__ n_active)
 {
-    __shared__ uint8_t in[2][kMcW + 1][kMcW + 4];  // y, z, x: the node is inside
-    const int i0 = (int)blockIdx.x * kMcW, j = (int)blockIdx.y, k0 = (int)blockIdx.z * kMcW;
-    for (int q = (int)threadIdx.x; q < 2 * (kMcW + 1) * (kMcW + 1); q += 256) {
-        const int i = q % (kMcW + 1), k = q / (kMcW + 1) % (kMcW + 1), y = q / ((kMcW + 1) * (kMcW + 1));
+    __shared__ uint8_t in[2][W + 1][kMcW + 4];  // y, z, x: the node is inside
+    const unsigned cubes = nb.x * nb.y * nb.z;
+    if (blockIdx.x >= cubes) {
+        const uint64_t t = g.cubes + (blockIdx.x - cubes) * (uint64_t)blockDim.x + threadIdx.x;
+        const bool on = t < items;
+        Item it{};
+        int cfg = 0;
+        if (on) {
+            it = decode(g, t);
+            cfg = cap_case(g, it.side, it.c);
+        }
+        count_item(g, on, t, it, cfg, cfg_out, nvert, ntri, active, n_active);
+        return;
+    }
+    const int i0 = (int)(blockIdx.x % nb.x) * kMcW, j = (int)(blockIdx.x / nb.x % nb.y), k0 = (int)(blockIdx.x / (nb.x * nb.y)) * W;
+    for (int q = (int)threadIdx.x; q < 2 * (W + 1) * (kMcW + 1); q += 256) {
+        const int i = q % (kMcW + 1), k = q / (kMcW + 1) % (W + 1), y = q / ((kMcW + 1) * (W + 1));
         if (i0 + i < g.n[0] && k0 + k < g.n[2]) in[y][k][i] = sdf_at(g, i0 + i, j + y, k0 + k) <= 0.0 ? 1 : 0;
     }
     __syncthreads();
-    const int k = (int)threadIdx.x & 31;
-    for (int i = (int)threadIdx.x >> 5; i < kMcW; i += 8) {
+    const int k = (int)threadIdx.x % W;
+    for (int i = (int)threadIdx.x / W; i < kMcW; i += 256 / W) {
         const bool on = i0 + i < g.n[0] - 1 && k0 + k < g.n[2] - 1;
         Item it;
         it.kind = 0;
@@ -242,23 +261,8 @@ __global__ void __launch_bounds__(256) k_mc_count_cubes(McGrid g, uint8_t* __res
                 constexpr int off[8][3] = FE_MC_CORNER_OFFSETS;
                 cfg |= in[off[v][1]][k + off[v][2]][i + off[v][0]] << v;
             }
-        count_item(g, on, on ? encode_cube(g, it.c[0], it.c[1], it.c[2]) : 0, it, cfg, cfg_out, nvert, ntri, active);
+        count_item(g, on, on ? encode_cube(g, it.c[0], it.c[1], it.c[2]) : 0, it, cfg, cfg_out, nvert, ntri, active, n_active);
     }
-}
-// The cap squares, an item a thread.
-__global__ void __launch_bounds__(256) k_mc_count_caps(McGrid g, uint64_t items, uint8_t* __restrict__ cfg_out,
-                                                       uint32_t* __restrict__ nvert, uint32_t* __restrict__ ntri,
-                                                       uint32_t* __restrict__ active)
-{
-    const uint64_t t = g.cubes + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    const bool on = t < items;
-    Item it{};
-    int cfg = 0;
-    if (on) {
-        it = decode(g, t);
-        cfg = cap_case(g, it.side, it.c);
-    }
-    count_item(g, on, t, it, cfg, cfg_out, nvert, ntri, active);
 }
 
 __device__ __forceinline__ double dm(double a, double b) { return __dmul_rn(a, b); }
@@ -439,16 +443,21 @@ McGrid mc_grid(const SceneView& v, const double* sdf)
 }  // namespace
 
 cudaError_t launch_mc_count(const SceneView& v, const double* sdf, uint8_t* cfg, uint32_t* nvert, uint32_t* ntri,
-                            uint32_t* active, cudaStream_t st)
+                            uint32_t* active, uint32_t* n_active, cudaStream_t st)
 {
     const McGrid g = mc_grid(v, sdf);
     const uint64_t items = mc_items(g.n[0], g.n[1], g.n[2]);
-    cudaError_t e = cudaMemsetAsync(active, 0, sizeof(uint32_t), st);
+    cudaError_t e = cudaMemsetAsync(n_active, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    k_mc_count_cubes<<<dim3((unsigned)((g.n[0] - 2) / kMcW + 1), (unsigned)(g.n[1] - 1), (unsigned)((g.n[2] - 2) / kMcW + 1)), 256,
-                       0, st>>>(g, cfg, nvert, ntri, active);
-    k_mc_count_caps<<<(unsigned)((items - g.cubes + 255) / 256), 256, 0, st>>>(g, items, cfg, nvert, ntri, active);
-    count_launch(2);
+    McCubeBlocks nb{(unsigned)((g.n[0] - 2) / kMcW + 1), (unsigned)(g.n[1] - 1), (unsigned)((g.n[2] - 2) / kMcW + 1)};
+    const unsigned caps = (unsigned)((items - g.cubes + 255) / 256);
+    if (nb.x * nb.y * nb.z < 2u * 148u) {
+        nb.z = (unsigned)((g.n[2] - 2) / 8 + 1);
+        k_mc_count<8><<<nb.x * nb.y * nb.z + caps, 256, 0, st>>>(g, nb, items, cfg, nvert, ntri, active, n_active);
+    } else {
+        k_mc_count<32><<<nb.x * nb.y * nb.z + caps, 256, 0, st>>>(g, nb, items, cfg, nvert, ntri, active, n_active);
+    }
+    count_launch();
     return cudaGetLastError();
 }
 
@@ -456,7 +465,7 @@ cudaError_t launch_mc_emit(const SceneView& v, const double* sdf, const uint32_t
                            const uint32_t* vbase, const uint32_t* tbase, double* V, double* N, int64_t* T, cudaStream_t st)
 {
     if (n_active == 0) return cudaSuccess;
-    k_mc_emit<<<(n_active + kMcEmit - 1) / kMcEmit, kMcEmit, 0, st>>>(mc_grid(v, sdf), active + 1, n_active, cfg, vbase, tbase, V, N,
+    k_mc_emit<<<(n_active + kMcEmit - 1) / kMcEmit, kMcEmit, 0, st>>>(mc_grid(v, sdf), active, n_active, cfg, vbase, tbase, V, N,
                                                                       T);
     count_launch();
     return cudaGetLastError();
