@@ -35,35 +35,6 @@
 namespace fe {
 namespace {
 
-// One CTA per triangle (grid-stride): the nodes of its index box take the minimum distance.
-__global__ void __launch_bounds__(256) k_mesh_band(MeshView m, NodeGrid g, unsigned long long* __restrict__ bits)
-{
-    const double inv = dd(1.0, g.h[0]);  // the reference scales every axis by 1 / h_x
-    for (uint64_t t = blockIdx.x; t < m.nt; t += gridDim.x) {
-        double p[3][3];
-        load_vertex(m, m.T[4 * t], p[0]);
-        load_vertex(m, m.T[4 * t + 1], p[1]);
-        load_vertex(m, m.T[4 * t + 2], p[2]);
-        int lo[3], hi[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const double f0 = dm(p[0][d], inv), f1 = dm(p[1][d], inv), f2 = dm(p[2][d], inv);
-            lo[d] = min(max((int)fmin(f0, fmin(f1, f2)) - 1, 0), g.n[d] - 1);
-            hi[d] = min(max((int)fmax(f0, fmax(f1, f2)) + 2, 0), g.n[d] - 1);
-        }
-        const int sx = hi[0] - lo[0] + 1, sy = hi[1] - lo[1] + 1, sz = hi[2] - lo[2] + 1;
-        const int64_t cells = (int64_t)sx * sy * sz;
-        for (int64_t q = threadIdx.x; q < cells; q += blockDim.x) {
-            const int i = lo[0] + (int)(q % sx), j = lo[1] + (int)((q / sx) % sy), k = lo[2] + (int)(q / ((int64_t)sx * sy));
-            const double pt[3] = {grid_pos(g, 0, i), grid_pos(g, 1, j), grid_pos(g, 2, k)};
-            const double d = distance_to_triangle(pt, p[0], p[1], p[2]);
-            const unsigned long long b = (unsigned long long)__double_as_longlong(d);
-            unsigned long long* cell = bits + idx3(i, j, k, g.n[0], g.n[1]);
-            if (b < __ldcg(cell)) atomicMin(cell, b);
-        }
-    }
-}
-
 // Whether the mesh is closed: every edge, as a pair of vertex positions, is used as often in one direction as in the
 // other.  Each use adds a hash of the undirected edge, with its direction as the sign, to two 64-bit sums, which are
 // zero for a closed mesh (and for an open one with probability 2^-128).  Then the solid angles of its triangles sum to
@@ -92,7 +63,7 @@ __device__ __forceinline__ int compare_points(const double p[3], const double q[
     }
     return 0;
 }
-__global__ void __launch_bounds__(256) k_mesh_closed(MeshView m, unsigned long long* __restrict__ state)
+__device__ __forceinline__ void mesh_edges(const MeshView& m, unsigned long long* state)
 {
     unsigned long long s0 = 0, s1 = 0;
     bool bad = false;
@@ -125,6 +96,37 @@ __global__ void __launch_bounds__(256) k_mesh_closed(MeshView m, unsigned long l
 __device__ __forceinline__ bool mesh_closed(const unsigned long long* state)
 {
     return (state[0] | state[1] | state[2]) == 0ull;
+}
+
+// One CTA per triangle (grid-stride): the nodes of its index box take the minimum distance; first the sums of the edges.
+__global__ void __launch_bounds__(256) k_mesh_band(MeshView m, NodeGrid g, unsigned long long* __restrict__ bits,
+                                                   unsigned long long* __restrict__ state)
+{
+    mesh_edges(m, state);
+    const double inv = dd(1.0, g.h[0]);  // the reference scales every axis by 1 / h_x
+    for (uint64_t t = blockIdx.x; t < m.nt; t += gridDim.x) {
+        double p[3][3];
+        load_vertex(m, m.T[4 * t], p[0]);
+        load_vertex(m, m.T[4 * t + 1], p[1]);
+        load_vertex(m, m.T[4 * t + 2], p[2]);
+        int lo[3], hi[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double f0 = dm(p[0][d], inv), f1 = dm(p[1][d], inv), f2 = dm(p[2][d], inv);
+            lo[d] = min(max((int)fmin(f0, fmin(f1, f2)) - 1, 0), g.n[d] - 1);
+            hi[d] = min(max((int)fmax(f0, fmax(f1, f2)) + 2, 0), g.n[d] - 1);
+        }
+        const int sx = hi[0] - lo[0] + 1, sy = hi[1] - lo[1] + 1, sz = hi[2] - lo[2] + 1;
+        const int64_t cells = (int64_t)sx * sy * sz;
+        for (int64_t q = threadIdx.x; q < cells; q += blockDim.x) {
+            const int i = lo[0] + (int)(q % sx), j = lo[1] + (int)((q / sx) % sy), k = lo[2] + (int)(q / ((int64_t)sx * sy));
+            const double pt[3] = {grid_pos(g, 0, i), grid_pos(g, 1, j), grid_pos(g, 2, k)};
+            const double d = distance_to_triangle(pt, p[0], p[1], p[2]);
+            const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+            unsigned long long* cell = bits + idx3(i, j, k, g.n[0], g.n[1]);
+            if (b < __ldcg(cell)) atomicMin(cell, b);
+        }
+    }
 }
 
 // Crossings of the grid rows along x with the triangles of a closed mesh, a warp per triangle, a lane per row.  cross[c]:
@@ -250,15 +252,13 @@ __global__ void __launch_bounds__(256) k_mesh_own(MeshView m, NodeGrid g, const 
     }
 }
 
-// TriangleMesh::IsInside at every node, then the signed value: -d inside, d outside.  k_mesh_rows: a closed mesh, a
+// TriangleMesh::IsInside at every node, then the signed value: -d inside, d outside.  mesh_rows: a closed mesh, a
 // warp per row, from the crossings (which share memory with the result: each lane reads its node's before it writes
 // it).  A node that sums for itself fixes the winding number for the nodes after it, unless it lies on the surface;
-// then the next one sums too, which the row's warp does where k_mesh_own has not.  k_mesh_sign: an open mesh, a thread per
+// then the next one sums too, which the row's warp does where k_mesh_own has not.  mesh_signs: an open mesh, a thread per
 // node.
-__global__ void __launch_bounds__(256) k_mesh_rows(MeshView m, NodeGrid g, const unsigned long long* __restrict__ state,
-                                                   const unsigned long long* __restrict__ bits, double* sdf)
+__device__ __forceinline__ void mesh_rows(const MeshView& m, const NodeGrid& g, const unsigned long long* bits, double* sdf)
 {
-    if (!mesh_closed(state)) return;
     const bool listed = mesh_listed(g);
     const int2* cross = reinterpret_cast<const int2*>(sdf);
     const int lane = threadIdx.x & 31;
@@ -314,10 +314,8 @@ __global__ void __launch_bounds__(256) k_mesh_rows(MeshView m, NodeGrid g, const
     }
 }
 
-__global__ void __launch_bounds__(256) k_mesh_sign(MeshView m, NodeGrid g, const unsigned long long* __restrict__ state,
-                                                   const unsigned long long* __restrict__ bits, double* __restrict__ sdf)
+__device__ __forceinline__ void mesh_signs(const MeshView& m, const NodeGrid& g, const unsigned long long* bits, double* sdf)
 {
-    if (m.nt && mesh_closed(state)) return;
     const double two_pi_tol = ds(dm(2.0, 3.14159265358979323846), 0.001);
     const size_t nc = (size_t)g.n[0] * g.n[1] * g.n[2];
     for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < nc; c += (size_t)gridDim.x * blockDim.x) {
@@ -328,9 +326,23 @@ __global__ void __launch_bounds__(256) k_mesh_sign(MeshView m, NodeGrid g, const
     }
 }
 
-__global__ void k_fill_bits(unsigned long long* __restrict__ bits, size_t n, unsigned long long v)
+// crossed: the crossings are recorded.
+__global__ void __launch_bounds__(256) k_mesh_finish(MeshView m, NodeGrid g, const unsigned long long* __restrict__ state, bool crossed,
+                                                     const unsigned long long* __restrict__ bits, double* sdf)
 {
-    for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) bits[c] = v;
+    if (crossed && mesh_closed(state)) mesh_rows(m, g, bits, sdf);
+    else mesh_signs(m, g, bits, sdf);
+}
+
+// No distance and no crossing yet, and nothing known of the mesh.
+__global__ void k_mesh_start(unsigned long long* __restrict__ bits, double* __restrict__ sdf, size_t n, unsigned long long v,
+                             unsigned long long* __restrict__ state)
+{
+    for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
+        bits[c] = v;
+        sdf[c] = 0.0;
+    }
+    if (blockIdx.x == 0 && threadIdx.x < kMeshStateWords) state[threadIdx.x] = 0ull;
 }
 
 __device__ __forceinline__ double uniform01(uint64_t seed, uint64_t counter)
@@ -449,28 +461,24 @@ cudaError_t launch_mesh_to_sdf(const double* V, uint64_t nv, const int64_t* T, u
     const double fill = hmax * (double)((size_t)n[0] + (size_t)n[1] + (size_t)n[2]);
     unsigned long long fill_bits;
     std::memcpy(&fill_bits, &fill, sizeof(fill_bits));
-    k_fill_bits<<<(unsigned)std::min<size_t>((nc + 255) / 256, 148 * 32), 256, 0, st>>>(scratch, nc, fill_bits);
+    MeshView m{V, T, nv, nv ? nt : 0};  // no vertices: no distances and no triangle to wind around (the fill stays positive)
+    k_mesh_start<<<(unsigned)std::min<size_t>((nc + 255) / 256, 148 * 32), 256, 0, st>>>(scratch, sdf, nc, fill_bits, state);
     count_launch();
-    MeshView m{V, T, nv, nt};
-    if (nv > 0 && nt > 0) {
-        k_mesh_band<<<(unsigned)std::min<uint64_t>(nt, 148 * 64), 256, 0, st>>>(m, g, scratch);
+    if (m.nt > 0) {
+        k_mesh_band<<<(unsigned)std::min<uint64_t>(nt, 148 * 64), 256, 0, st>>>(m, g, scratch, state);
         count_launch();
     }
-    if (nv == 0) m.nt = 0;  // no vertices: no distances and no triangle to wind around (the fill stays positive)
-    if (m.nt > 0) {
-        // the closed path's kernels and the open path's look at the sums and leave what is not theirs
-        cudaError_t e = cudaMemsetAsync(state, 0, kMeshStateWords * sizeof(unsigned long long), st);
-        if (e != cudaSuccess) return e;
-        if ((e = cudaMemsetAsync(sdf, 0, nc * sizeof(double), st)) != cudaSuccess) return e;
-        k_mesh_closed<<<(unsigned)std::min<uint64_t>((nt + 255) / 256, 148 * 8), 256, 0, st>>>(m, state);
-        k_mesh_cross<<<(unsigned)std::min<uint64_t>((nt + 7) / 8, 148 * 8), 256, 0, st>>>(m, g, state,
-                                                                                         reinterpret_cast<int2*>(sdf));
+    // a node's winding terms take 0.6 us a triangle, and all nodes' 1 us for some 10^5: sums that are through sooner than the two
+    // passes that save them (some 28 us) are taken directly (a call, with / without the passes: 20 triangles on 32^3 nodes 275 /
+    // 259 us, 80 on 16^3 209 / 255, 320 on 16^3 230 / 455)
+    const bool crossed = m.nt >= 48 || (double)m.nt * (double)nc >= 3.0 * (1 << 20);
+    if (crossed) {
+        k_mesh_cross<<<(unsigned)std::min<uint64_t>((nt + 7) / 8, 148 * 8), 256, 0, st>>>(m, g, state, reinterpret_cast<int2*>(sdf));
         k_mesh_own<<<148 * 8, 256, 0, st>>>(m, g, state, reinterpret_cast<int2*>(sdf));
-        k_mesh_rows<<<(unsigned)std::min<size_t>(((size_t)n[1] * n[2] + 7) / 8, 148 * 32), 256, 0, st>>>(m, g, state, scratch,
-                                                                                                       sdf);
-        count_launch(4);
+        count_launch(2);
     }
-    k_mesh_sign<<<(unsigned)std::min<size_t>((nc + 255) / 256, 148 * 32), 256, 0, st>>>(m, g, state, scratch, sdf);
+    const size_t blocks = std::max((nc + 255) / 256, ((size_t)n[1] * n[2] + 7) / 8);
+    k_mesh_finish<<<(unsigned)std::min<size_t>(blocks, 148 * 32), 256, 0, st>>>(m, g, state, crossed, scratch, sdf);
     count_launch();
     return cudaGetLastError();
 }

@@ -60,3 +60,14 @@ def test_not_slower_than_an_open_mesh(n, cells):
         return min(times)
 
     assert best(T) <= 2.0 * best(T[:-1])
+
+
+@pytest.mark.parametrize("n", [(16, 16, 16), (65, 64, 64), (7, 90, 4)])
+@pytest.mark.parametrize("cells", [1, 2, 3])
+def test_few_triangles(n, cells):
+    """12 and 48 triangles: either side of the counts from which crossings are recorded; closed and open."""
+    h = 1.0 / 32
+    V, T = box(n, h, cells)
+    V = V * 0.77 + 0.01  # off the nodes
+    for triangles in (T, T[:-1]):
+        assert np.array_equal(fe.mesh_to_sdf(V, triangles, n, ZERO, (h,) * 3), oracle.mesh_to_sdf(V, triangles, n, ZERO, (h,) * 3))
