@@ -488,8 +488,8 @@ def batched_measure(n_scenes=48, steps=50, warmup=5, device=0, batch_family=None
     8 particles per cell, solver drawn from PIC / FLIP(0.95) / APIC (seed 2).  Both arms use the same
     pressure tolerance (rel 1e-6); times are wall clock around synchronised device work.  The one-at-a-time arm
     runs every scene with the autotuner's choice for its kind, and so does the batched arm by default;
-    batch_family="cg" runs the batched arm's scenes on the plain CG body inside the multi-scene solve instead (with
-    the current multigrid solver slower for this set: 12.29 against 11.31 ms per substep).  Returns a dict.
+    batch_family="cg" runs the batched arm's scenes on the plain CG body inside the multi-scene solve instead (9.38
+    against 7.48 ms per substep for this set).  Returns a dict.
     """
     import numpy as np
     import torch

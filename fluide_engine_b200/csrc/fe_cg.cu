@@ -257,12 +257,10 @@ __global__ void __launch_bounds__(kMultiThreads, 3) k_multi_cg(MultiCgScene* __r
     }
 }
 
-// Relative cost of one inner iteration per FLUID cell: the multigrid body's passes and grid barriers (4 L - 2 per
-// iteration) against the plain body's one.
 __device__ __forceinline__ double multi_work(const MultiCgScene& m)
 {
     if (m.last_its < 0) return m.weight0;
-    const double per_it = m.use_mg ? 12.0 : 1.0;
+    const double per_it = m.use_mg ? kMultigridIterationWork : 1.0;
     return (double)m.last_fluid * ((double)m.last_its * per_it + 3.0);
 }
 

@@ -323,7 +323,8 @@ constexpr int kMaxMgLevels = 12;
 // FE_PRESSURE_AUTO picks the multigrid solver from this many grid cells on (grids of at most 8 cells per axis have no
 // hierarchy and keep the plain one).  Measured on B200, dam break to 1e-6 (us per solve, plain / multigrid): 12^3 211 /
 // 178, 16^3 285 / 190, 20^3 348 / 244, 24^3 426 / 266, 28^3 479 / 258, 32^3 539 / 256, 40^3 635 / 309; 64^3 and above the
-// plain one takes two to ten times as long.
+// plain one takes two to ten times as long.  Fluid one or two cells deep needs few plain iterations (4 x 40 x 40 cells, 1.6 of them
+// deep: 143 / 256; 16 x 24: 590 / 324, full 722 / 332): the size alone does not tell, and the plain one loses more.
 constexpr size_t kMgAutoCells = (size_t)1 << 10;
 struct MgLevel {
     int nx, ny, nz;
@@ -358,6 +359,11 @@ struct MultiCgScene {
     int last_its, last_fluid;      // the previous solve's inner iterations and FLUID cells (-1 / 0: none yet)
     double weight0;                // expected solve work before any solve has run
 };
+// Work of one inner iteration of the multigrid body per FLUID cell, the plain body's being 1, by which the blocks are split
+// among scenes that use one or the other.  ms a solve at 4 / 9 / 12 / 18 / 27: 15 pools of 32^3 .. 128^3, two thirds plain, 19.8 /
+// 14.3 / 14.3 / 14.7 / 15.0; 12 dams of 32^3 .. 96^3, half plain, 1.45 / 1.41 / 1.51 / 1.73 / 2.21; a plain 64^3 beside two of
+// 96^3 1.20 / 1.28 / 1.30 / 1.51 / 1.77.
+constexpr double kMultigridIterationWork = 12.0;
 cudaError_t multi_cg_capacity(int device, int* max_blocks, int* threads);
 // Re-splits total_blocks among the S scenes in proportion to their last solve's work, then solves them.
 cudaError_t launch_multi_cg(MultiCgScene* scenes, int S, int total_blocks, cudaStream_t st);

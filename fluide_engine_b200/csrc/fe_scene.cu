@@ -3127,7 +3127,7 @@ fe_status batch_resplit(fe_batch* b)
     double total = 0.0;
     for (int i = 0; i < S; ++i) {
         const MultiCgScene& m = table[i];
-        const double per_it = m.use_mg ? 12.0 : 1.0;
+        const double per_it = m.use_mg ? kMultigridIterationWork : 1.0;
         work[i] = m.last_its >= 0 ? (double)m.last_fluid * ((double)m.last_its * per_it + 3.0) : m.weight0;
         work[i] = std::max(work[i], 0.0);
         total += work[i];
