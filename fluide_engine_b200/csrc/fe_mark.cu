@@ -212,6 +212,7 @@ struct MarkShared {
 // holds, a 128^3 FLIP dam break after 480 substeps, 1600 to 2000 particles in its fullest cell, took 172 us here (one pass over the
 // particles 112), now 46.
 constexpr uint32_t kNearLanesCap = 64;
+constexpr int kNearThreads = 256;
 __device__ __forceinline__ void mark_near_body(const SceneView& v, const MarkConst& mc, int tile, MarkShared& sh)
 {
     const uint32_t first = (uint32_t)tile * FE_TILE_CELLS;
@@ -239,14 +240,16 @@ __device__ __forceinline__ void mark_near_body(const SceneView& v, const MarkCon
         }
     }
     __syncthreads();
-    const int n = sh.count;
-    for (int e = (int)(threadIdx.x >> 3); e < n; e += (int)(blockDim.x >> 3)) {
-        const uint32_t key = first + sh.list[e];
-        for (uint32_t p = v.cell_start[key] + (threadIdx.x & 7), pe = v.cell_start[key + 1]; p < pe; p += 8) mark_particle(v, mc, p);
-    }
-    for (int e = 0, m = sh.crowded; e < m; ++e) {
-        const uint32_t key = first + sh.list[FE_TILE_CELLS - 1 - e];
-        for (uint32_t p = v.cell_start[key] + threadIdx.x, pe = v.cell_start[key + 1]; p < pe; p += blockDim.x) mark_particle(v, mc, p);
+    // one loop for both kinds of cell (with two calls of mark_particle 6 us more at 128^3)
+#pragma unroll 1
+    for (int lg = 3; lg <= 8; lg += 5) {  // 8 lanes, then the block's 256
+        const int n = lg == 3 ? sh.count : sh.crowded;
+        for (int e = (int)threadIdx.x >> lg; e < n; e += kNearThreads >> lg) {
+            const uint32_t key = first + sh.list[lg == 3 ? e : FE_TILE_CELLS - 1 - e];
+            const uint32_t step = 1u << lg;
+            for (uint32_t p = v.cell_start[key] + (threadIdx.x & (step - 1u)), pe = v.cell_start[key + 1]; p < pe; p += step)
+                mark_particle(v, mc, p);
+        }
     }
 }
 
@@ -350,7 +353,7 @@ __device__ __forceinline__ void mark_fixup_body(const SceneView& v, double R2, u
 __global__ void k_mark_fixup(SceneView v, double R2, uint32_t cap) { mark_fixup_body(v, R2, cap, blockIdx.x, gridDim.x); }
 
 __global__ void __launch_bounds__(256) k_mark_own(SceneView v, MarkConst mc) { mark_own_body(v, mc, blockIdx.x); }
-__global__ void __launch_bounds__(256) k_mark_near(SceneView v, MarkConst mc)
+__global__ void __launch_bounds__(kNearThreads) k_mark_near(SceneView v, MarkConst mc)
 {
     __shared__ MarkShared sh;
     mark_near_body(v, mc, (int)blockIdx.x, sh);
@@ -834,7 +837,7 @@ cudaError_t launch_mark(const SceneView& v, bool cells_current, cudaStream_t st)
         const unsigned nb = (unsigned)((v.np + 255) / 256);
         if (mc.two && cells_current && v.np >= (v.any_inexact ? kMarkTwoPassesInexact : kMarkTwoPasses)) {
             k_mark_own<<<nb, 256, 0, st>>>(v, mc);
-            k_mark_near<<<(unsigned)(v.g.tnx * v.g.tny * v.g.tnz), 256, 0, st>>>(v, mc);
+            k_mark_near<<<(unsigned)(v.g.tnx * v.g.tny * v.g.tnz), kNearThreads, 0, st>>>(v, mc);
             count_launch(2);
         } else {
             k_mark<<<nb, 256, 0, st>>>(v, mc);

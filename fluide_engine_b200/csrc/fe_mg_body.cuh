@@ -933,7 +933,7 @@ __device__ __forceinline__ void mg_body(MgShared& ms, MgTeam* __restrict__ teams
                             }
                             diag += C.ih2[a] * coef;
                         }
-                    if (inner) diag += kInnerAir * (C.ih2[0] + C.ih2[1] + C.ih2[2]) * sqrtf(fmaxf(1.f - own, 0.f));
+                    if (inner && own < 1.f) diag += kInnerAir * (C.ih2[0] + C.ih2[1] + C.ih2[2]) * sqrtf(1.f - own);
                     inv = diag > 0.f ? 1.f / diag : 0.f;
                 }
                 C.inv[c] = inv;
