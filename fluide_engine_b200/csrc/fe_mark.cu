@@ -536,8 +536,7 @@ struct NodeShared {
     uint16_t row[kNodeHalo * kNodeHaloZ];  // occupied cells of a row, a bit each
     uint8_t near[FE_TILE * kNodeLayers];   // nodes of a row with an occupied cell that reaches into their band
     uint16_t list[kNodeThreads];           // nodes to search, a thread each
-    uint16_t hard[kNodeThreads];           // ... the crowded cells, a warp each
-    double best[kNodeThreads];             // of those: the smallest squared distance in the other cells
+    uint16_t hard[kNodeThreads];           // ... the crowded cells, a warp each; `out` holds the others' smallest squared distance
     double near2[kNodeCells];
     int16_t cell[kNodeCells];              // offset in start and count
     int n, nhard;
@@ -697,11 +696,8 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
                 else full = true;
             }
         }
-        if (full) {
-            const int e = atomicAdd(&sh.nhard, 1);
-            sh.hard[e] = (uint16_t)t;
-            sh.best[e] = best;
-        } else out[idx3(i, j, k, nx, ny)] = value(best);
+        if (full) sh.hard[atomicAdd(&sh.nhard, 1)] = (uint16_t)t;
+        out[idx3(i, j, k, nx, ny)] = full ? best : value(best);
     }
     __syncthreads();
 
@@ -718,7 +714,7 @@ __global__ void __launch_bounds__(kNodeThreads, 4) k_sdf_gather(SceneView v, con
         const int lx = t & 7, ly = (t >> 3) & 7, lz = t >> 6;
         const int i = x0 + lx, j = y0 + ly, k = z0 + lz;
         const double qx = v.q_pos[0][i], qy = v.q_pos[1][j], qz = v.q_pos[2][k];
-        double best = sh.best[e];
+        double best = out[idx3(i, j, k, nx, ny)];  // in the other cells
         for (int first = 0; first < kNodeCells; first += 32) {  // each lane looks at a cell
             const int c = first + lane;
             uint32_t s = 0, n = 0;
