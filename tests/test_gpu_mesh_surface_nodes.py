@@ -65,7 +65,7 @@ def test_not_slower_than_an_open_mesh(n, cells):
 @pytest.mark.parametrize("n", [(16, 16, 16), (65, 64, 64), (7, 90, 4)])
 @pytest.mark.parametrize("cells", [1, 2, 3])
 def test_few_triangles(n, cells):
-    """12 and 48 triangles: either side of the counts from which crossings are recorded; closed and open."""
+    """12, 48 and 108 triangles: either side of the counts from which crossings are recorded; closed and open."""
     h = 1.0 / 32
     V, T = box(n, h, cells)
     V = V * 0.77 + 0.01  # off the nodes
